@@ -80,7 +80,7 @@ static int series_len(const int* off, const int* type, int n, int want_type) {
 static Layout make_layout(const af_case_desc* c, const af_forcing_desc* f, double t_stop, int R,
                           int esize) {
   Layout L;
-  const int N = 16 / esize;
+  const int N = lane_cols(esize);
   L.nx = c->nx;
   L.ny = c->ny;
   L.P = row_pitch(c->nx, N);
@@ -281,7 +281,7 @@ static int create(int precision, int device, uint64_t arena_bytes, int variant, 
   b->device = device;
   b->prec = precision;
   b->esize = precision == AF_PREC_F64 ? 8 : 4;
-  b->N = 16 / b->esize;
+  b->N = lane_cols(b->esize);
   if (variant < 0) {
     // Default: 1 warp per block with 16 resident blocks per SM in FP32 (128
     // registers, no spills: the fastest shape on every measured mix), 12 in
@@ -428,6 +428,7 @@ static int add(Batch& b, const af_case_desc* c, const af_forcing_desc* f, const 
   p.dx = c->dx;
   p.dxinv = 1.0 / c->dx;  // src/kernels.cpp:8
   p.dA = c->dx * c->dx;   // src/main.cpp:115
+  set_reciprocals(p);
   p.fpn = c->fpn;
   p.depth_thresh = c->depth_thresh;
   p.max_hflow = c->max_hflow;

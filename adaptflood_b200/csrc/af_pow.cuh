@@ -195,5 +195,52 @@ AF_POW_HD double pow_ref(double x, double y) {
 #endif
 }
 
+#ifdef __CUDACC__
+// x^(10/3) for 2^-30 <= x <= 2^30: pow_ref's table path, operation by
+// operation, without its tests (y log x is below 70 and, unless x = 1, above
+// 2^-54; at x = 1 the table path gives 1 as well).
+__device__ __forceinline__ double pow_depth(double x) {
+  const double y = 10.0 / 3.0;
+  // log_hilo
+  const int xh = __double2hiint(x);
+  const int tmp = xh - (int)(AF_POW_OFF >> 32);  // AF_POW_OFF's low word is 0
+  const LogEntry le = log_entry((tmp >> 13) & 127);
+  const double z = __hiloint2double(xh - (tmp & 0xfff00000), __double2loint(x));
+  // (double)(tmp >> 20) by a sum with 2^52 (exact), not the conversion unit
+  const double kd = __hiloint2double(0x43300000, (tmp >> 20) + 2048) - (0x1p52 + 2048.0);
+  const double r = __fma_rn(z, le.invc, -1.0);
+  const double t1 = __fma_rn(kd, AF_POW_LN2HI, le.logc);
+  const double t2 = t1 + r;
+  const double lo1 = __fma_rn(kd, AF_POW_LN2LO, le.logctail);
+  const double lo2 = t1 - t2 + r;
+  const double ar = AF_POW_A0 * r;
+  const double ar2 = r * ar;
+  const double ar3 = r * ar2;
+  const double hi0 = t2 + ar2;
+  const double lo3 = __fma_rn(ar, r, -ar2);
+  const double lo4 = t2 - hi0 + ar2;
+  const double q = __fma_rn(ar2, __fma_rn(ar2, __fma_rn(r, AF_POW_A6, AF_POW_A5), __fma_rn(r, AF_POW_A4, AF_POW_A3)),
+                            __fma_rn(r, AF_POW_A2, AF_POW_A1));
+  const double lo = __fma_rn(ar3, q, lo1 + lo2 + lo3 + lo4);
+  const double hi = hi0 + lo;
+  const double tail = hi0 - hi + lo;
+  const double ehi = y * hi;
+  const double elo = __fma_rn(y, tail, __fma_rn(y, hi, -ehi));
+  // exp_hilo
+  const double ks = __fma_rn(AF_POW_INVLN2N, ehi, AF_POW_SHIFT);
+  const int ki = __double2loint(ks);
+  const double k = ks - AF_POW_SHIFT;
+  double s = __fma_rn(k, AF_POW_NEGLN2LON, __fma_rn(k, AF_POW_NEGLN2HIN, ehi));
+  s += elo;
+  const ExpEntry ee = exp_entry(ki & 127);
+  const double s2 = s * s;
+  const double s4 = s2 * s2;
+  const double w = __fma_rn(s4, __fma_rn(s, AF_POW_C5, AF_POW_C4),
+                            __fma_rn(s2, __fma_rn(s, AF_POW_C3, AF_POW_C2), as_double(ee.tail) + s));
+  const double scale = __hiloint2double((int)(ee.sbits >> 32) + (ki << 13), (int)(uint32_t)ee.sbits);
+  return __fma_rn(scale, w, scale);
+}
+#endif
+
 }  // namespace pw
 }  // namespace af

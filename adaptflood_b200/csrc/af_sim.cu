@@ -232,11 +232,10 @@ __global__ void k_gather(const T* __restrict__ H, int nx, int P, const int* __re
 struct Sim {
   int device = 0;
   int prec = AF_PREC_F64;
-  int esize = 8, N = 2;
+  int esize = 8, N = 1;
   cudaStream_t st = nullptr;
   af_case_desc c{};
   int P = 0, nsx = 0, nsy = 0, R = 16, WY = 4, variant = 0;
-  bool face_call = false;  // FP64: the step kernel with out-of-line faces
   bool tma = true;         // the step kernel reads rows with tiled copies
   size_t cells_elems = 0, qy_elems = 0;  // field sizes (elements, guards included)
   // The fields are planes of one allocation, each qy_elems long, in the order
@@ -275,22 +274,24 @@ struct Sim {
 
 // The step kernel of the simulation's precision, shape and face evaluation.
 static const void* step_fn(const Sim& s) {
-  return s.prec == AF_PREC_F64 ? step_kernel_f64(s.variant, s.face_call, s.tma)
+  return s.prec == AF_PREC_F64 ? step_kernel_f64(s.variant, s.tma)
                                : step_kernel_f32(s.variant, s.tma);
 }
 
 static int pick_shape(Sim& s) {
   const int own = 30 * s.N;
   s.nsx = (s.c.nx + own - 1) / own;
-  // Launch shape: FP32 one-warp blocks, 16 per SM (120 registers); FP64 20 per
-  // SM (96 registers: measured 6 % faster than 16 per SM on the 8192^2 step).
-  s.variant = s.prec == AF_PREC_F64 ? 2 : 0;
+  // Launch shape: FP32 one-warp blocks, 16 per SM (120 registers).  FP64 is
+  // compiled for 12 per SM, which gives its face law's two chains room to
+  // overlap (126 registers; 16 blocks are resident all the same): ms per step
+  // against the forms compiled for 16 and for 20, 8192^2 1.587 / 1.658 /
+  // 1.625, 2731x2747 0.215 / 0.221 / 0.215.
+  s.variant = s.prec == AF_PREC_F64 ? 1 : 0;
   if (const char* v = getenv("AF_SIM_VARIANT")) {
     const int k = atoi(v);
     if (k >= 0 && k < kStepVariants) s.variant = k;
   }
   s.WY = kStepVariant[s.variant].wy;
-  s.face_call = face_call_for(s.prec == AF_PREC_F64, (long long)s.c.nx * s.c.ny);
   s.tma = tma_for(s.prec == AF_PREC_F64, (long long)s.c.nx * s.c.ny);
   const void* fn = step_fn(s);
   int per_sm = 0, dev = 0, sms = kSMs;
@@ -310,18 +311,19 @@ static int pick_shape(Sim& s) {
   // strips fill at most two waves of the resident blocks takes the shortest
   // strips that still fit in as many waves, so every block gets the same
   // number of strips and each is as short as it can be (measured against
-  // powers of two: 512^2 +21 %, 2048^2 +6 %, 4096^2 +5 %).  The FP64 step,
-  // bound by its arithmetic, keeps more, shorter strips on mid-size grids
-  // (measured 8-9 % faster than the two-wave rule at 2048^2 and 4096^2), and
-  // on grids of up to 2^20 cells (less than one wave) two-row strips, the
-  // shortest serial chain per warp (512^2: 34.7 ms for the 1442-step C1 run
-  // against 50.2 ms with four rows).
+  // powers of two: 512^2 +21 %, 2048^2 +6 %, 4096^2 +5 %).  The FP64 step is
+  // bound by its arithmetic, so its strips (30 columns wide) are as tall as
+  // still leaves several waves of them: us per step at the chosen height and
+  // its neighbours, 512^2 R4 22.2 (R2 23.0, R6 21.8), 1024^2 R8 43.2 (R4 45.8,
+  // R12 45.0), 1501x1100 R8 60.0 (R4 66.0, R16 61.3), 2731x2747 R24 196 (R8
+  // 215, R32 198), 4096^2 R32 414 (R16 437, R48 422).
   const long long cells = (long long)s.c.nx * s.c.ny;
   s.R = 32;
   if (s.prec == AF_PREC_F64) {
-    if (cells <= (1LL << 20)) s.R = 2;
-    else if (cells <= (1LL << 23)) s.R = 8;
-    else if (cells <= (1LL << 25)) s.R = 16;
+    if (cells <= (1LL << 19)) s.R = 4;
+    else if (cells <= (1LL << 21)) s.R = 8;
+    else if (cells <= (1LL << 22)) s.R = 16;
+    else if (cells <= (1LL << 23)) s.R = 24;
   } else if (cells < (1LL << 20)) {
     // Small FP32 grids: one-row strips, the shortest chain per warp even at
     // slightly over one wave (ms per step, one row against the two-wave rule:
@@ -602,7 +604,7 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   s->device = device;
   s->prec = precision;
   s->esize = precision == AF_PREC_F64 ? 8 : 4;
-  s->N = 16 / s->esize;
+  s->N = lane_cols(s->esize);
   s->c = *c;
   s->case_hash = case_hash(c, f);
   AF_CUDA(cudaSetDevice(device));
@@ -686,6 +688,7 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   p.dx = c->dx;
   p.dxinv = 1.0 / c->dx;  // src/kernels.cpp:8
   p.dA = c->dx * c->dx;   // src/main.cpp:115
+  set_reciprocals(p);
   p.fpn = c->fpn;
   p.depth_thresh = c->depth_thresh;
   p.max_hflow = c->max_hflow;

@@ -14,6 +14,7 @@
 // Padding is zero and never read into an owned result.
 #pragma once
 
+#include <cmath>
 #include <vector>
 
 #include "af_step.cuh"
@@ -31,6 +32,14 @@ inline int row_pitch(int nx, int N) {
 // Elements of a cell field and of the Qy field, guards included.
 inline size_t cell_elems(int ny, int P) { return (size_t)kGuard * 2 + (size_t)ny * P; }
 inline size_t qy_elems(int ny, int P) { return (size_t)kGuard * 2 + (size_t)(ny + 1) * P; }
+
+// 1/dx and 1/dA to twice the precision (see div_const): lo = (1 - d*hi)/d,
+// the bracket exact in one fma.
+inline void set_reciprocals(StepParams& p) {
+  p.dxinv_lo = std::fma(-p.dx, p.dxinv, 1.0) / p.dx;
+  p.dAinv = 1.0 / p.dA;
+  p.dAinv_lo = std::fma(-p.dA, p.dAinv, 1.0) / p.dA;
+}
 
 inline bool non_decreasing(const double* t, int n) {
   for (int i = 0; i + 1 < n; i++)

@@ -10,8 +10,8 @@
 // the volume and flooded area (src/main.cpp:291-304).
 //
 // Work decomposition ("strips"): a warp owns OWN = 30*N consecutive columns
-// and R consecutive rows and marches down the rows.  Its 32 lanes each load N
-// consecutive cells (one 16-byte vector: N = 2 doubles or 4 floats) of every
+// and R consecutive rows and marches down the rows.  Its 32 lanes each take N
+// consecutive cells (one double, or one 16-byte vector of 4 floats) of every
 // array; lanes 0 and 31 are halo lanes whose cells belong to the neighbouring
 // warps, so every x-neighbour a face needs is one warp shuffle away and the
 // warp never touches shared memory.  Each face flux is computed by the lane
@@ -37,7 +37,7 @@
 #include <cstdlib>
 
 #include "af_common.cuh"
-#include "af_pow.cuh"
+#include "af_face64.cuh"
 
 // FP32 face-law experiments: AF_FRICTION 1 evaluates the friction factors
 // correctly rounded; AF_FACE_FORM 1 forms the flow depth and the head
@@ -102,6 +102,7 @@ struct StepParams {
   int nx, ny, P;      // grid and row pitch (elements)
   int nsx, nsy, R;    // strips in x and y, rows per strip
   double dx, dxinv, dA, fpn, depth_thresh, max_hflow, g, cfl, init_tstep, nodata;
+  double dxinv_lo, dAinv, dAinv_lo;  // 1/dx = dxinv + dxinv_lo, 1/dA = dAinv + dAinv_lo
   double mass_int;
   int wf, ef, nf, sf;
   int has_nodata;  // some DEM cell (as stored) equals nodata; 0 lets FP32 skip the tests
@@ -137,7 +138,7 @@ template <typename T>
 struct Lanes;
 template <>
 struct Lanes<double> {
-  static constexpr int N = 2;
+  static constexpr int N = 1;
 };
 template <>
 struct Lanes<float> {
@@ -149,9 +150,10 @@ __device__ inline T gmaxT(T a, T b) { return (a > b) ? a : b; }  // src/types.hp
 template <typename T>
 __device__ inline T gminT(T a, T b) { return (a < b) ? a : b; }  // src/types.hpp:15
 
-__device__ inline void st_vec(double* p, const double (&v)[2]) {
-  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-}
+// Columns per lane of a precision given by its element size.
+inline int lane_cols(int esize) { return esize == 8 ? Lanes<double>::N : Lanes<float>::N; }
+
+__device__ inline void st_vec(double* p, const double (&v)[1]) { *p = v[0]; }
 __device__ inline void st_vec(float* p, const float (&v)[4]) {
   *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -161,6 +163,8 @@ struct Phys {
   T dx, fn, depth_thresh, max_hflow, nodata, gdt;  // gdt = g*dt
   T g;
   T dxinv, gdt_fn2;  // 1/dx and g*dt*fn*fn/dx (FP32 form only)
+  T rh, rl, ah, al;  // 1/dx as rh + rl and 1/dA as ah + al (FP64 form only)
+  bool fast;         // the step's constants are in face_fast's range (FP64 form only)
 };
 
 // FREE edges (src/kernels.cpp:154-248).  West also needs the cell east of
@@ -264,83 +268,35 @@ __device__ inline T bc_depth(int b, SeriesTable tb, double t) {
 // `if (Q*dh < 0)` recomputation (src/kernels.cpp:86-89) yields the same Q
 // (both numerators are equal whenever Q != 0), so it is not repeated.
 
-// The FP64 wet-face expression out of line (the same results), for the step
-// kernel of mid-size grids: the four inline copies per row of a lane make the
-// row loop's code large enough to stall on instruction fetch.  Measured, ms
-// per step out of line against inline: 724^2 0.0714 / 0.0823, 1024^2 0.106 /
-// 0.124, 2048^2 0.247 / 0.269, 4096^2 0.676 / 0.716, 5793^2 1.222 / 1.265;
-// level at 512^2 (one wave of strips) and 6896^2, and on 8192^2 inline is
-// faster (2.22 against 2.32: the four faces' chains overlap in the FP64 pipe).
-static __device__ __noinline__ double face_q64(double dh, double hflow, double q0, double qa, double qb,
-                                        double qc, double qd, double dx, double gdt, double fn) {
-  const double Sf = -dh / dx;
+// One FP64 face with every test of the reference (src/kernels.cpp:56-92), out
+// of line: the face row above a strip, and rows where face_fast found an
+// operand out of its range.
+static __device__ __noinline__ double face_any64(double z0, double h0, double z1, double h1,
+                                                 double q0, double qa, double qb, double qc,
+                                                 double qd, bool enable, bool fast, double dx,
+                                                 double rh, double rl, double gdt, double fn,
+                                                 double depth_thresh, double max_hflow,
+                                                 double nodata) {
+  if (!enable | (z0 == nodata) | (z1 == nodata)) return 0.0;
+  const double y0 = z0 + h0, y1 = z1 + h1;
+  double hflow = gmaxT(y0, y1) - gmaxT(z0, z1);
+  hflow = gmaxT(hflow, 0.0);
+  hflow = gminT(hflow, max_hflow);
+  if (!(hflow > depth_thresh)) return 0.0;
+  const double dh = y0 - y1;
   const double qy_avg = (qa + qb + qc + qd) / 4.0;
-  const double qvect = sqrt(q0 * q0 + qy_avg * qy_avg);
+  const double x = q0 * q0 + qy_avg * qy_avg;
+  if (fast) {
+    bool bad;
+    const double q = face_fast(dh, hflow, x, q0, dx, rh, rl, gdt, fn, bad);
+    if (!bad) return q;
+  }
+  const double Sf = -dh / dx;
+  const double qvect = sqrt(x);
   const double numerator = (q0 + 0.0) - (gdt * hflow * Sf);
   const double denominator =
       1.0 + gdt * hflow * fn * fn * fabs(qvect) / pw::pow_ref(hflow, 10.0 / 3.0);
   return numerator / denominator * dx;
-}
-
-// FP64: the reference's expressions exactly (src/kernels.cpp:60-84), with the
-// C library's pow algorithm (af_pow.cuh).
-template <bool ND, bool kCall = false>  // FP64 keeps every test of the reference
-__device__ inline void row_faces(const double (&h)[2], const double (&z)[2], const double (&hN)[2],
-                                 const double (&zN)[2], const double (&qxo)[2],
-                                 const double (&qxoN)[2], const double (&qyo)[2],
-                                 const double (&qyoN)[2], double hL, double zL, double qyoL,
-                                 double qyoNL, double qxoR, double qxoNR, bool south,
-                                 const Phys<double>& ph, double (&qw)[2], double (&qs)[2]) {
-  double Z0[4], H0[4], Z1[4], H1[4], Q0[4], QA[4], QB[4], QC[4], QD[4];
-  // faces 0,1: west faces of cells 0,1; faces 2,3: south faces of cells 0,1
-  Z0[0] = zL;   H0[0] = hL;   Z1[0] = z[0]; H1[0] = h[0];
-  Q0[0] = qxo[0]; QA[0] = qyoL; QB[0] = qyo[0]; QC[0] = qyoNL; QD[0] = qyoN[0];
-  Z0[1] = z[0]; H0[1] = h[0]; Z1[1] = z[1]; H1[1] = h[1];
-  Q0[1] = qxo[1]; QA[1] = qyo[0]; QB[1] = qyo[1]; QC[1] = qyoN[0]; QD[1] = qyoN[1];
-  Z0[2] = z[0]; H0[2] = h[0]; Z1[2] = zN[0]; H1[2] = hN[0];
-  Q0[2] = qyoN[0]; QA[2] = qxo[0]; QB[2] = qxo[1]; QC[2] = qxoN[0]; QD[2] = qxoN[1];
-  Z0[3] = z[1]; H0[3] = h[1]; Z1[3] = zN[1]; H1[3] = hN[1];
-  Q0[3] = qyoN[1]; QA[3] = qxo[1]; QB[3] = qxoR; QC[3] = qxoN[1]; QD[3] = qxoNR;
-  double y0[4], y1[4], hf[4];
-  bool wet[4];
-  bool any = false;
-#pragma unroll
-  for (int f = 0; f < 4; f++) {
-    y0[f] = Z0[f] + H0[f];
-    y1[f] = Z1[f] + H1[f];
-    double hflow = gmaxT(y0[f], y1[f]) - gmaxT(Z0[f], Z1[f]);
-    hflow = gmaxT(hflow, 0.0);
-    hflow = gminT(hflow, ph.max_hflow);
-    hf[f] = hflow;
-    wet[f] = (f < 2 || south) && !(Z0[f] == ph.nodata || Z1[f] == ph.nodata) &&
-             hflow > ph.depth_thresh;
-    any |= wet[f];
-  }
-  double Q[4] = {0.0, 0.0, 0.0, 0.0};
-  if (__any_sync(0xffffffffu, any)) {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const double dh = y0[f] - y1[f];
-      double q;
-      if constexpr (kCall) {
-        q = face_q64(dh, hf[f], Q0[f], QA[f], QB[f], QC[f], QD[f], ph.dx, ph.gdt, ph.fn);
-      } else {
-        const double Sf = -dh / ph.dx;
-        const double hflow = hf[f];
-        const double qy_avg = (QA[f] + QB[f] + QC[f] + QD[f]) / 4.0;
-        const double qvect = sqrt(Q0[f] * Q0[f] + qy_avg * qy_avg);
-        const double numerator = (Q0[f] + 0.0) - (ph.gdt * hflow * Sf);
-        const double denominator =
-            1.0 + ph.gdt * hflow * ph.fn * ph.fn * fabs(qvect) / pw::pow_ref(hflow, 10.0 / 3.0);
-        q = numerator / denominator * ph.dx;
-      }
-      Q[f] = wet[f] ? q : 0.0;
-    }
-  }
-  qw[0] = Q[0];
-  qw[1] = Q[1];
-  qs[0] = Q[2];
-  qs[1] = Q[3];
 }
 
 // FP32: the same face law on pairs of faces with Blackwell's packed FP32x2
@@ -422,7 +378,7 @@ __device__ inline float2 flux2(float2 z0, float2 h0, float2 z1, float2 h1, float
   return f2(wx ? __fdividef(num.x, den.x) : 0.0f, wy ? __fdividef(num.y, den.y) : 0.0f);
 }
 
-template <bool ND, bool kCall = false>  // kCall: FP64 only
+template <bool ND>
 __device__ inline void row_faces(const float (&h)[4], const float (&z)[4], const float (&hN)[4],
                                  const float (&zN)[4], const float (&qxo)[4],
                                  const float (&qxoN)[4], const float (&qyo)[4],
@@ -473,7 +429,15 @@ constexpr int kStages = AF_STAGES;  // ring depth (rows in flight per warp, incl
 #define AF_EDGE_SPLIT 1
 #endif
 constexpr int kRowUnroll = AF_ROW_UNROLL;
-constexpr int kRowBytes = 512;
+// A row's window: 32 lanes x N columns, and in FP64 (N = 1) two columns more
+// on each side to start at a 16-byte boundary and fill whole 128-byte units
+// per stage: 36 columns from x0 - 2.
+template <typename T>
+struct RowWin {
+  static constexpr int lead = sizeof(T) == 8 ? 1 : 0;  // columns left of lane 0's
+  static constexpr int cols = sizeof(T) == 8 ? 36 : 128;
+  static constexpr int bytes = cols * (int)sizeof(T);
+};
 constexpr long long kWaitLimit = 1LL << 22;
 // Polls a warp spends waiting for a row of its ring before it gives up (the
 // drain after a give-up keeps kWaitLimit).  A test build sets it to 0, so
@@ -541,10 +505,8 @@ __device__ inline void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-__device__ inline void lds_vec(const unsigned char* p, double (&v)[2]) {
-  const double2 t = *reinterpret_cast<const double2*>(p);
-  v[0] = t.x;
-  v[1] = t.y;
+__device__ inline void lds_vec(const unsigned char* p, double (&v)[1]) {
+  v[0] = *reinterpret_cast<const double*>(p);
 }
 __device__ inline void lds_vec(const unsigned char* p, float (&v)[4]) {
   const float4 t = *reinterpret_cast<const float4*>(p);
@@ -567,31 +529,44 @@ struct BoolC {
 // would round it the same way in every cell of a binade (a bias in the
 // volume), while the flux term differs from cell to cell.  The reference's
 // clamp between rain and update has no effect there (rain >= 0, depth >= 0).
-template <bool ND>  // FP64 keeps every test of the reference
-__device__ inline void update_cells(double (&hn)[2], const double (&qw)[2], const double (&qe)[2],
-                                    const double (&qn)[2], const double (&qs)[2],
-                                    const double (&z)[2], bool rain_on, double rain_depth,
-                                    double dt, double dA, double /*dt_dA*/, double nodata) {
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    double v = hn[k];
-    if (rain_on && z[k] != nodata) {
-      v = v + rain_depth;
-      if (v < 0.0) v = 0.0;
-    }
-    v = v + dt * (qw[k] - qe[k] + qn[k] - qs[k]) / dA;
-    if (v < 0.0) v = 0.0;
-    hn[k] = v;
+// Rare pieces of the FP64 row loop, out of line so that the loop stays short
+// and none of their work is done ahead of the branch that needs it.
+static __device__ __noinline__ double div_any64(double a, double b) { return a / b; }
+static __device__ __noinline__ double out_free64(double h, double z, double sign, double g,
+                                                 double dx, double nodata) {
+  return out_free(h, z, sign, g, dx, nodata);
+}
+static __device__ __noinline__ double west_free64(double h0, double z0, double h1, double z1,
+                                                  double g, double dx, double nodata) {
+  return west_free(h0, z0, h1, z1, g, dx, nodata);
+}
+
+__device__ inline double update_cell(double h, double qw, double qe, double qn, double qs,
+                                     bool rain, double rain_depth, double dt, double dA,
+                                     const Phys<double>& ph) {
+  const double w = dt * (qw - qe + qn - qs);
+  double dv = div_const(w, dA, ph.ah, ph.al);
+  const int wh = __double2hiint(w) & 0x7fffffff;
+  if (!ph.fast | (((unsigned)(wh - ((1023 - 900) << 20)) >= (unsigned)(1800 << 20)) &
+                  ((wh | __double2loint(w)) != 0)))
+    dv = div_any64(w, dA);
+  if (rain) {
+    h = h + rain_depth;
+    if (h < 0.0) h = 0.0;
   }
+  h = h + dv;
+  if (h < 0.0) h = 0.0;
+  return h;
 }
 template <bool ND>
 __device__ inline void update_cells(float (&hn)[4], const float (&qw)[4], const float (&qe)[4],
                                     const float (&qn)[4], const float (&qs)[4],
                                     const float (&z)[4], bool rain_on, float rain_depth,
-                                    float /*dt*/, float /*dA*/, float dt_dA, float nodata) {
+                                    float /*dt*/, float /*dA*/, float dt_dA,
+                                    const Phys<float>& ph) {
   float rk[4];
 #pragma unroll
-  for (int k = 0; k < 4; k++) rk[k] = (rain_on && (!ND || z[k] != nodata)) ? rain_depth : 0.0f;
+  for (int k = 0; k < 4; k++) rk[k] = (rain_on && (!ND || z[k] != ph.nodata)) ? rain_depth : 0.0f;
 #pragma unroll
   for (int k = 0; k < 4; k += 2) {
     const float2 a = __ffma2_rn(f2(qe[k], qe[k + 1]), f2(-1.0f, -1.0f), f2(qw[k], qw[k + 1]));
@@ -645,6 +620,11 @@ __device__ inline void fill_scalars(const StepParams& p, double t, double dt, do
   s.ph.gdt = T(p.g * dt);  // (g*dt) rounded once, as the reference's left-to-right product does
   s.ph.dxinv = T(1.0 / p.dx);
   s.ph.gdt_fn2 = T(p.g * dt * p.fpn * p.fpn * p.dxinv);
+  s.ph.rh = T(p.dxinv);
+  s.ph.rl = T(p.dxinv_lo);
+  s.ph.ah = T(p.dAinv);
+  s.ph.al = T(p.dAinv_lo);
+  s.ph.fast = face_range_ok(p.dx, p.fpn, p.depth_thresh, p.max_hflow, p.g * dt);
 }
 
 template <typename T>
@@ -678,7 +658,7 @@ struct LaneAcc {
   __device__ bool any_cell() const { return m_cell != T(-FLT_MAX); }
 };
 
-// One step of strip (sx, sy) of one grid by one warp: the strip's OWN
+// One FP32 step (FP64: run_strip64) of strip (sx, sy) of one grid by one warp: the strip's OWN
 // columns and R rows, streamed through the warp's stage ring (`ring`, `bar`;
 // `pos` = the warp's position in the ring, advanced past the strip's stages).
 // Warps whose strip lies wholly inside the grid in x take a path without the
@@ -686,27 +666,23 @@ struct LaneAcc {
 // copies in flight drained and the grid's status flagged.
 // kSplitND: FP32 grids without nodata cells take a copy of the row loop
 // without the nodata tests (the same results; the batch kernel uses it, the
-// single-grid kernel measured no faster with it).  kCall: FP64 evaluates each
-// wet face out of line (see face_q64).
+// single-grid kernel measured no faster with it).
 // kTma: one tiled copy per row through `tmap` instead of four bulk copies.
-template <typename T, bool kSplitND = false, bool kCall = false, bool kTma = false>
+template <typename T, bool kSplitND = false, bool kTma = false>
 __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>& sc, int sx,
-                                          int sy, unsigned char (*ring)[4][kRowBytes],
+                                          int sy, unsigned char (*ring)[4][RowWin<T>::bytes],
                                           uint64_t* bar, RingPos& pos, LaneAcc<T>& acc,
                                           const CUtensorMap* tmap = nullptr) {
   constexpr int N = Lanes<T>::N;
   constexpr int OWN = 30 * N;
-  static_assert(32 * N * sizeof(T) == kRowBytes, "one 16-byte vector per lane");
-  // FP64 forms the reference's Qold = Q*(1/dx) on load (its exact rounding);
-  // the FP32 face law works on Q itself (1/dx folded into its coefficients).
-  constexpr bool kQold = Lanes<T>::N == 2;
+  constexpr int kRowBytes = RowWin<T>::bytes;
+  static_assert(sizeof(T) == 4, "the face law here works on Q itself (1/dx in its coefficients)");
   const int lane = threadIdx.x & 31;
   const int nx = p.nx, ny = p.ny, P = p.P;
   const int parity = sc.parity;
   const double t = sc.t, dt = sc.dt;
   const bool mass = sc.mass, rain_on = sc.rain_on;
-  const T rain_depth = sc.rain_depth, dtT = sc.dtT, dAT = sc.dAT, dxinvT = sc.dxinvT,
-          dt_dA = sc.dt_dA;
+  const T rain_depth = sc.rain_depth, dtT = sc.dtT, dAT = sc.dAT, dt_dA = sc.dt_dA;
   const Phys<T> ph = sc.ph;
   const T* __restrict__ H = static_cast<const T*>(p.H[parity]);
   T* __restrict__ Hn = static_cast<T*>(p.H[parity ^ 1]);
@@ -719,7 +695,7 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
 
   const int x0 = sx * OWN;
   const int cb = x0 - N + lane * N;          // first column of this lane
-  const long long wcol = (long long)x0 - N;  // first column of the warp's window
+  const long long wcol = (long long)x0 - N - RowWin<T>::lead;  // first column of the window
   const bool own = lane >= 1 && lane <= 30;
   const int j0 = sy * p.R;
   const int j1 = min(j0 + p.R, ny);
@@ -800,7 +776,7 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
   int kc = 0;  // next stage of this strip to consume, at ring position `pos`
   auto acquire = [&]() -> const unsigned char* {
     if (!mbar_wait_warp(&bar[pos.slot()], pos.phase(), kRingWaitLimit)) return nullptr;
-    return &ring[pos.slot()][0][0] + lane * 16;
+    return &ring[pos.slot()][0][0] + (lane * N + RowWin<T>::lead) * (int)sizeof(T);
   };
   // The consumed stage is refilled with the row kStages ahead (same slot).
   auto release = [&]() {
@@ -831,13 +807,6 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
       lds_vec(st + 2 * kRowBytes, qxo);
       lds_vec(st + 3 * kRowBytes, qyo);
       release();
-#pragma unroll
-      for (int k = 0; k < N; k++) {
-        if (kQold) {
-          qxo[k] = qxo[k] * dxinvT;
-          qyo[k] = qyo[k] * dxinvT;
-        }
-      }
     }
   }
   if (!failed) {
@@ -859,9 +828,6 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
       // strip above uses to compute and store them, so both strips see the
       // same flux through their common edge, bit for bit, in either
       // precision.  The west faces it also returns are not needed here.
-#pragma unroll
-      for (int k = 0; k < N; k++)
-        if (kQold) qxp[k] = qxp[k] * dxinvT;
       const T qxpR = __shfl_down_sync(0xffffffffu, qxp[0], 1);
       const T qxoR = __shfl_down_sync(0xffffffffu, qxo[0], 1);
       T qw_unused[N];
@@ -870,10 +836,9 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
     }
   }
 
-  auto rows = [&](auto edge_tag, auto nd_tag, auto call_tag) {
+  auto rows = [&](auto edge_tag, auto nd_tag) {
     constexpr bool kEdge = decltype(edge_tag)::value;
     constexpr bool kND = decltype(nd_tag)::value;
-    constexpr bool kFaceCall = decltype(call_tag)::value;
 #pragma unroll kRowUnroll
     for (int j = j0; j < j1; j++) {
       const bool has_next = (j + 1 < ny);
@@ -894,13 +859,6 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
           for (int k = 0; k < N; k++) hN[k] = zN[k] = qxoN[k] = T(0);
         }
         release();
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-          if (kQold) {
-            qyoN[k] = qyoN[k] * dxinvT;
-            qxoN[k] = qxoN[k] * dxinvT;
-          }
-        }
       }
       // Neighbours across lanes.
       const T hL = __shfl_up_sync(0xffffffffu, h[N - 1], 1);
@@ -912,8 +870,7 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
 
       // Faces of the row: interior law everywhere, then the edges.
       T qw[N], qs[N];
-      row_faces<kND, kFaceCall>(h, z, hN, zN, qxo, qxoN, qyo, qyoN, hL, zL, qyoL, qyoNL, qxoR,
-                                qxoNR,
+      row_faces<kND>(h, z, hN, zN, qxo, qxoN, qyo, qyoN, hL, zL, qyoL, qyoNL, qxoR, qxoNR,
                      has_next, ph, qw, qs);
       if (kEdge) {
 #pragma unroll
@@ -969,7 +926,7 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
         sp++;
         next_row = sp < sp_end ? p.spec[sp].row : INT_MAX;
       }
-      update_cells<kND>(hn, qw, qe, qyn, qs, z, rain_on, rain_depth, dtT, dAT, dt_dA, ph.nodata);
+      update_cells<kND>(hn, qw, qe, qyn, qs, z, rain_on, rain_depth, dtT, dAT, dt_dA, ph);
       // Point depth BCs (src/kernels.cpp:259-277), after the update.
       for (int q = sp_row; q < sp; q++) {
         const SpecCell e = p.spec[q];
@@ -1029,22 +986,22 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
     }
   };
   if (!failed) {
-    // FP32 takes a copy of the row loop without nodata tests on grids that
-    // have no nodata cell; FP64 keeps the reference's tests everywhere.
+    // Grids that have no nodata cell may take a copy of the row loop without
+    // nodata tests.
     bool nd = true;
-    if constexpr (sizeof(T) == 4 && kSplitND) nd = p.has_nodata != 0;
+    if constexpr (kSplitND) nd = p.has_nodata != 0;
 #if AF_EDGE_SPLIT
     const bool interior = (x0 > 0) && (x0 + OWN < nx);
 #else
     const bool interior = false;
 #endif
     if (nd) {
-      if (interior) rows(BoolC<false>(), BoolC<true>(), BoolC<kCall>());
-      else rows(BoolC<true>(), BoolC<true>(), BoolC<kCall>());
+      if (interior) rows(BoolC<false>(), BoolC<true>());
+      else rows(BoolC<true>(), BoolC<true>());
     } else {
       if constexpr (kSplitND) {
-        if (interior) rows(BoolC<false>(), BoolC<false>(), BoolC<false>());
-        else rows(BoolC<true>(), BoolC<false>(), BoolC<false>());
+        if (interior) rows(BoolC<false>(), BoolC<false>());
+        else rows(BoolC<true>(), BoolC<false>());
       }
     }
   }
@@ -1058,6 +1015,246 @@ __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>
       d.advance();
     }
     for (int k = kc; k < nload; k++) pos.advance();  // past the strip's stages
+    if (lane == 0) atomicExch(&p.ctl->status, 2);
+  }
+  return !failed;
+}
+
+// The FP64 form of run_strip.  A lane owns one column (30 per strip), so the
+// row loop holds two faces, straight-line and interleaved (af_face64.cuh);
+// the step is bound by instruction issue and the FP64 pipe (2.64 of 4
+// instructions per cycle and 47 % at 4096^2; DRAM 25 %), and a longer loop
+// loses to instruction fetch: with two columns and four faces per lane the
+// loop issues 13 % fewer instructions per cell but stalls on fetch three
+// times as often and is slower up to 4096^2 (2731x2747 0.252 ms per step
+// against 0.216), level at 8192^2; unrolled by two it takes 0.329.  So one
+// copy of the loop serves interior and edge strips (edge work behind a branch
+// the whole warp takes or not), and rare work is out of line.  The left
+// neighbour's bed and depth come from the stage (its column is in the
+// window), and what a row needs of its neighbours is kept for the next one.
+// us per step, before (library division, square root and pow per face) and
+// now: 1501x1100 127 / 60, 2731x2747 333 / 196, 8192^2 2151 / 1587.
+template <bool kTma>
+__device__ __forceinline__ bool run_strip64(const StepParams& p, const StepScal<double>& sc, int sx,
+                                            int sy, unsigned char (*ring)[4][RowWin<double>::bytes],
+                                            uint64_t* bar, RingPos& pos, LaneAcc<double>& acc,
+                                            const CUtensorMap* tmap = nullptr) {
+  constexpr int OWN = 30;
+  constexpr int kRowBytes = RowWin<double>::bytes;
+  int lane;  // read once: not recomputed from the thread index in the loop
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  const int nx = p.nx, ny = p.ny, P = p.P;
+  const int parity = sc.parity;
+  const double dxinv = sc.dxinvT;
+  const Phys<double> ph = sc.ph;
+  const int x0 = sx * OWN;
+  const int c = x0 - 1 + lane;  // this lane's column
+  const int wcol = x0 - 1 - RowWin<double>::lead;
+  const int j0 = sy * p.R;
+  const int j1 = min(j0 + p.R, ny);
+  const bool own = lane >= 1 && lane <= 30 && c < nx;
+  const bool edge = x0 == 0 || x0 + OWN >= nx;  // the strip holds a west or east edge face
+  const int strip = sx * p.nsy + sy;
+  int sp = p.spec_off[strip];
+  const int sp_end = p.spec_off[strip + 1];
+  int next_row = sp < sp_end ? p.spec[sp].row : INT_MAX;
+  const int rfirst = j0 > 0 ? j0 - 1 : j0;
+  const int nload = j1 + 1 - rfirst;
+  const uint32_t row_bytes =
+      (uint32_t)min(kRowBytes, ((nx + 1 - wcol) * (int)sizeof(double) + 15) & ~15);
+  const double* const my_src =
+      static_cast<const double*>(lane == 0   ? p.H[parity]
+                                 : lane == 1 ? p.DEM
+                                 : lane == 2 ? p.Qx[parity]
+                                             : p.Qy[parity]);
+  auto issue = [&](int k, int slot) {
+    const int r = rfirst + k;
+    if constexpr (kTma) {
+      if (lane == 0) {
+        mbar_expect_tx(&bar[slot], 4u * kRowBytes);
+        fence_proxy_async();
+        tma_load_3d(&ring[slot][0][0], tmap, wcol, r, 4 * parity, &bar[slot]);
+      }
+    } else {
+      const int a_lo = r < ny ? 0 : 3;
+      const int a_hi = r < j0 ? 3 : 4;
+      if (lane == 0) mbar_expect_tx(&bar[slot], (uint32_t)(a_hi - a_lo) * row_bytes);
+      if (lane >= a_lo && lane < a_hi) {
+        fence_proxy_async();
+        bulk_g2s(&ring[slot][lane][0], my_src + (long long)r * P + wcol, row_bytes, &bar[slot]);
+      }
+    }
+  };
+  {
+    RingPos f = pos;
+    for (int k = 0; k < kStages && k < nload; k++) {
+      issue(k, f.slot());
+      f.advance();
+    }
+  }
+  __syncwarp();
+  int kc = 0;
+  bool failed = false;
+  // The row at the ring's position: this lane's cell and faces, its left
+  // neighbour's bed and depth; then the stage is refilled.
+  double hN, zN, qxN, qyN, hNL, zNL;
+  auto take = [&]() -> bool {
+    if (!mbar_wait_warp(&bar[pos.slot()], pos.phase(), kRingWaitLimit)) return false;
+    const double* st = reinterpret_cast<const double*>(&ring[pos.slot()][0][0]) + lane;
+    constexpr int W = RowWin<double>::cols;
+    hNL = st[0];
+    hN = st[1];
+    zNL = st[W];
+    zN = st[W + 1];
+    qxN = st[2 * W + 1];
+    qyN = st[3 * W + 1];
+    __syncwarp();
+    if (kc + kStages < nload) issue(kc + kStages, pos.slot());
+    kc++;
+    pos.advance();
+    qxN = qxN * dxinv;  // Qold (src/kernels.cpp:8-16)
+    qyN = qyN * dxinv;
+    return true;
+  };
+  double h = 0.0, z = 0.0, zL = 0.0, y = 0.0, yL = 0.0, qx = 0.0, qy = 0.0, qn = 0.0;
+  double hp = 0.0, zp = 0.0, qxp = 0.0;
+  if (j0 > 0) {
+    failed = !take();
+    hp = hN;
+    zp = zN;
+    qxp = qxN;
+  }
+  if (!failed) failed = !take();
+  double qyL = 0.0, qxR = 0.0;
+  bool v = true, vL = true;
+  if (!failed) {
+    h = hN;
+    z = zN;
+    zL = zNL;
+    y = zN + hN;
+    yL = zNL + hNL;
+    qx = qxN;
+    qy = qyN;
+    qyL = __shfl_up_sync(0xffffffffu, qy, 1);
+    qxR = __shfl_down_sync(0xffffffffu, qx, 1);
+    v = z != ph.nodata;
+    vL = zL != ph.nodata;
+    if (j0 == 0) {
+      if (p.nf) qn = out_free64(h, z, -1.0, ph.g, ph.dx, ph.nodata);
+      if (own) static_cast<double*>(p.Qy[parity ^ 1])[c] = qn;
+    } else {
+      const double qxpR = __shfl_down_sync(0xffffffffu, qxp, 1);
+      qn = face_any64(zp, hp, z, h, qy, qxp, qxpR, qx, qxR, true, ph.fast, ph.dx, ph.rh, ph.rl,
+                      ph.gdt, ph.fn, ph.depth_thresh, ph.max_hflow, ph.nodata);
+    }
+  }
+  // Rows of the new state, advanced row by row (Qy: the row below).
+  double* Hn = static_cast<double*>(p.H[parity ^ 1]) + (long long)j0 * P;
+  double* Qxn = static_cast<double*>(p.Qx[parity ^ 1]) + (long long)j0 * P;
+  double* Qyn = static_cast<double*>(p.Qy[parity ^ 1]) + (long long)(j0 + 1) * P;
+#pragma unroll 1
+  for (int j = j0; j < j1 && !failed; j++, Hn += P, Qxn += P, Qyn += P) {
+    // Past the last row only Qy is copied; the rest of the stage reaches only
+    // the south face, which is masked there.
+    if (!take()) {
+      failed = true;
+      break;
+    }
+    const bool south = j + 1 < ny;
+    const double yN = zN + hN, yNL = zNL + hNL;
+    const double qyNL = __shfl_up_sync(0xffffffffu, qyN, 1);
+    const double qxNR = __shfl_down_sync(0xffffffffu, qxN, 1);
+    const bool vN = zN != ph.nodata, vNL = zNL != ph.nodata;
+    // West and south face.  The reference's clamp of the flow depth at 0 only
+    // matters for a threshold below 0, which is not `fast`.
+    const double hw = gminT(gmaxT(yL, y) - gmaxT(zL, z), ph.max_hflow);
+    const double hs = gminT(gmaxT(y, yN) - gmaxT(z, zN), ph.max_hflow);
+    const bool wet_w = v & vL & (hw > ph.depth_thresh);
+    const bool wet_s = v & vN & south & (hs > ph.depth_thresh);
+    double qw = 0.0, qs = 0.0;
+    if (__any_sync(0xffffffffu, wet_w | wet_s | !ph.fast)) {
+      const double aw = (qyL + qy + qyNL + qyN) / 4.0, as = (qx + qxR + qxN + qxNR) / 4.0;
+      bool bw, bs;
+      const double fw = face_fast(yL - y, hw, qx * qx + aw * aw, qx, ph.dx, ph.rh, ph.rl, ph.gdt,
+                                  ph.fn, bw);
+      const double fs = face_fast(y - yN, hs, qyN * qyN + as * as, qyN, ph.dx, ph.rh, ph.rl, ph.gdt,
+                                  ph.fn, bs);
+      qw = wet_w ? fw : 0.0;
+      qs = wet_s ? fs : 0.0;
+      if (__any_sync(0xffffffffu, (bw & wet_w) | (bs & wet_s) | !ph.fast)) {
+        const double hL = __shfl_up_sync(0xffffffffu, h, 1);
+        qw = face_any64(zL, hL, z, h, qx, qyL, qy, qyNL, qyN, true, ph.fast, ph.dx, ph.rh, ph.rl,
+                        ph.gdt, ph.fn, ph.depth_thresh, ph.max_hflow, ph.nodata);
+        qs = face_any64(z, h, zN, hN, qyN, qx, qxR, qxN, qxNR, south, ph.fast, ph.dx, ph.rh, ph.rl,
+                        ph.gdt, ph.fn, ph.depth_thresh, ph.max_hflow, ph.nodata);
+      }
+    }
+    if (!south) qs = p.sf ? out_free64(h, z, 1.0, ph.g, ph.dx, ph.nodata) : 0.0;
+    if (edge) {
+      const double h1 = __shfl_down_sync(0xffffffffu, h, 1);
+      const double z1 = __shfl_down_sync(0xffffffffu, z, 1);
+      if (c == 0) qw = p.wf ? west_free64(h, z, h1, z1, ph.g, ph.dx, ph.nodata) : 0.0;
+    }
+    double qe = __shfl_down_sync(0xffffffffu, qw, 1);
+    if (edge && c == nx - 1) {
+      qe = p.ef ? out_free64(h, z, 1.0, ph.g, ph.dx, ph.nodata) : 0.0;
+      if (own) Qxn[c + 1] = qe;
+    }
+    // Point sources (src/main.cpp:245-262), before rain and the update.
+    double hn = h;
+    const int sp_row = sp;
+    while (next_row == j) {
+      const SpecCell e = p.spec[sp];
+      if (own && e.col == c)
+        hn = apply_sources(hn, e.s0, e.s1,
+                           SeriesTable{p.src_type, p.src_value, p.src_off, p.src_times, p.src_vals,
+                                       p.src_sorted},
+                           p.dx, p.dA, sc.t, sc.dt);
+      sp++;
+      next_row = sp < sp_end ? p.spec[sp].row : INT_MAX;
+    }
+    hn = update_cell(hn, qw, qe, qn, qs, sc.rain_on & v, sc.rain_depth, sc.dtT, sc.dAT, ph);
+    // Point depth BCs (src/kernels.cpp:259-277), after the update.
+    for (int q = sp_row; q < sp; q++) {
+      const SpecCell e = p.spec[q];
+      if (own && e.bc >= 0 && e.col == c)
+        hn = bc_depth<double>(e.bc,
+                              SeriesTable{p.bc_type, p.bc_value, p.bc_off, p.bc_times, p.bc_vals,
+                                          p.bc_sorted},
+                              sc.t);
+    }
+    if (own) {
+      Hn[c] = hn;
+      Qxn[c] = qw;
+      Qyn[c] = qs;
+      if (v) acc.m_cell = (hn > acc.m_cell) ? hn : acc.m_cell;  // a NaN never wins
+      if (__builtin_expect(sc.mass, 0)) {
+        acc.v += hn * p.dA;
+        if (hn > 0.01) acc.a += p.dA;
+      }
+    }
+    h = hN;
+    z = zN;
+    zL = zNL;
+    y = yN;
+    yL = yNL;
+    qx = qxN;
+    qy = qyN;
+    qyL = qyNL;
+    qxR = qxNR;
+    v = vN;
+    vL = vNL;
+    qn = qs;
+  }
+  if (failed) {
+    // Drain the copies still in flight (bounded) and flag the control block.
+    const int issued = min(nload, kc + kStages);
+    RingPos d = pos;
+    for (int k = kc; k < issued; k++) {
+      mbar_wait_warp(&bar[d.slot()], d.phase());
+      d.advance();
+    }
+    for (int k = kc; k < nload; k++) pos.advance();
     if (lane == 0) atomicExch(&p.ctl->status, 2);
   }
   return !failed;
@@ -1108,16 +1305,16 @@ __device__ inline bool fold_step(const StepParams& p, SimCtl* ctl, double t, dou
 // strip sx).  The last block to finish folds the step.  kTma: rows are read
 // with one tiled copy per row through the tensor map `fields` (the grid's
 // fields as planes of one 3-D tensor); otherwise four bulk copies per row.
-template <typename T, int WY, int MINB, bool kCall = false, bool kTma = true>
+template <typename T, int WY, int MINB, bool kTma = true>
 __global__ void __launch_bounds__(32 * WY, MINB) k_step(const StepParams p,
                                                         const __grid_constant__ CUtensorMap fields) {
-  __shared__ __align__(128) unsigned char s_ring[WY][kStages][4][kRowBytes];
+  __shared__ __align__(128) unsigned char s_ring[WY][kStages][4][RowWin<T>::bytes];
   __shared__ __align__(8) uint64_t s_bar[WY][kStages];
   SimCtl* ctl = p.ctl;
   if (*(volatile int*)&ctl->done) return;
 
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
+  const int warp = WY == 1 ? 0 : threadIdx.x >> 5;
   StepScal<T> sc;
   step_scalars(p, ctl->t, ctl->hmax, ctl->rain_rate, ctl->next_mass, ctl->parity, sc);
   const bool mass = sc.mass;
@@ -1135,8 +1332,12 @@ __global__ void __launch_bounds__(32 * WY, MINB) k_step(const StepParams p,
     const int sx = tile % p.nsx;
     const int sy = (tile / p.nsx) * WY + warp;
     if (sy >= p.nsy) continue;
-    if (!run_strip<T, false, kCall, kTma>(p, sc, sx, sy, s_ring[warp], bar, pos, acc, &fields))
-      break;
+    bool ok;
+    if constexpr (sizeof(T) == 8)
+      ok = run_strip64<kTma>(p, sc, sx, sy, s_ring[warp], bar, pos, acc, &fields);
+    else
+      ok = run_strip<T, false, kTma>(p, sc, sx, sy, s_ring[warp], bar, pos, acc, &fields);
+    if (!ok) break;
   }
 
   // A valid cell's depth is finite (NaN never wins a comparison), and in
@@ -1468,7 +1669,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_batch_fold(const BatchParams b
 
 template <typename T, int WY, int MINB>
 __global__ void __launch_bounds__(32 * WY, MINB) k_batch_step(const BatchParams bp) {
-  __shared__ __align__(128) unsigned char s_ring[WY][kStages][4][kRowBytes];
+  __shared__ __align__(128) unsigned char s_ring[WY][kStages][4][RowWin<T>::bytes];
   __shared__ __align__(8) uint64_t s_bar[WY][kStages + 1];  // the ring's, then the records'
   __shared__ BatchScen s_rec[WY][2];
   if (*(volatile int*)&bp.bctl->done) return;
@@ -1544,7 +1745,10 @@ __global__ void __launch_bounds__(32 * WY, MINB) k_batch_step(const BatchParams 
     const StepScal<T>& sc = *reinterpret_cast<const StepScal<T>*>(rec.scal);
     const int k = u - tab->u0[a];
     LaneAcc<T> acc{T(-FLT_MAX), 0.0, 0.0};
-    ok = run_strip<T, true>(p, sc, k % p.nsx, k / p.nsx, s_ring[warp], bar, pos, acc);
+    if constexpr (sizeof(T) == 8)
+      ok = run_strip64<false>(p, sc, k % p.nsx, k / p.nsx, s_ring[warp], bar, pos, acc);
+    else
+      ok = run_strip<T, true>(p, sc, k % p.nsx, k / p.nsx, s_ring[warp], bar, pos, acc);
     double m = acc.any_cell() ? (double)acc.m_cell : -DBL_MAX;
     m = warp_maxd(m);
     double v = 0.0, ar = 0.0;
@@ -1577,17 +1781,6 @@ __global__ void __launch_bounds__(32 * WY, MINB) k_batch_step(const BatchParams 
   if (!ok && lane == 0) atomicExch(&bp.bctl->status, 1);
 }
 
-// Whether a single grid's FP64 step takes the kernel that evaluates each wet
-// face out of line (k_step<double, ..., true>): on grids of more than 2^18
-// and at most 2^25 cells (see face_q64).  AF_SIM_FACE_CALL=0/1 forces the
-// choice (for measurements).
-constexpr long long kFaceCallMinCells = (1LL << 18) + 1;
-constexpr long long kFaceCallMaxCells = 1LL << 25;
-inline bool face_call_for(bool f64, long long cells) {
-  if (!f64) return false;
-  if (const char* v = getenv("AF_SIM_FACE_CALL")) return v[0] == '1';
-  return cells >= kFaceCallMinCells && cells <= kFaceCallMaxCells;
-}
 // Whether a single grid's step reads its rows with one tiled copy (TMA) per
 // row instead of four bulk copies: FP32 grids of at most kTmaMaxCellsF32
 // cells, FP64 grids of at most kTmaMaxCellsF64.  The tiled copies take fewer
@@ -1630,7 +1823,7 @@ inline int encode_field_planes(CUtensorMap* out, void* origin, int esize, int nx
   }
   const cuuint64_t dims[3] = {(cuuint64_t)nx + 1, (cuuint64_t)ny + 1, 8};
   const cuuint64_t strides[2] = {(cuuint64_t)P * esize, (cuuint64_t)plane_bytes};
-  const cuuint32_t box[3] = {(cuuint32_t)(kRowBytes / esize), 1, 4};
+  const cuuint32_t box[3] = {(cuuint32_t)(esize == 8 ? RowWin<double>::cols : RowWin<float>::cols), 1, 4};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode(
       out, esize == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
@@ -1647,7 +1840,7 @@ struct StepVariant {
 };
 constexpr int kStepVariants = 5;
 constexpr StepVariant kStepVariant[kStepVariants] = {{1, 16}, {1, 12}, {1, 20}, {4, 4}, {2, 8}};
-const void* step_kernel_f64(int variant, bool face_call = false, bool tma = true);
+const void* step_kernel_f64(int variant, bool tma = true);
 const void* step_kernel_f32(int variant, bool tma = true);
 const void* batch_kernel_f64(int variant);
 const void* batch_kernel_f32(int variant);
