@@ -1,0 +1,805 @@
+// af_resident.cuh -- the time loop of a small grid in one launch, its state
+// held on chip.
+//
+// A step of a small grid costs a kernel boundary, a prologue of dependent
+// loads and one trip to L2 per row, not bandwidth: 64 k cells took 11.4 us a
+// step and 0.8 M cells 20 us, against 0.3 and 3.4 us of HBM time.  Here one
+// cooperative launch runs all the steps of a call: block b of (at most) one
+// per SM keeps a band of rows in shared memory and exchanges with the others
+// only its first and last rows' new H and Qx and its Hmax.
+//
+// Exchange.  Every 8 bytes that cross blocks carry 4 bytes of data and the
+// step's tag, so a reader polls the data itself and no fence, flag or atomic
+// stands between a step's last store and the next step's first use (an
+// 8-byte aligned access is not torn).  Buffers alternate between two copies:
+// a block writes step n+2's only after it has read every block's Hmax of
+// step n+1, which each sends after it has read step n's.  All blocks derive
+// the same dt, time and loop decisions from the same Hmax, so nothing else is
+// shared.  Every wait is bounded; a block that gives up flags the control
+// block and leaves, and so then do the others.
+//
+// Work.  A warp marches 32 columns down some rows, as the strip kernels do but
+// without halo lanes: the left neighbours come from shared memory, and the
+// faces on the strip's east side, for all its rows at once (a lane each),
+// share one evaluation with the faces above its first row.  The same face
+// law, edge law and update functions as the strip kernels, in the same order,
+// so results are the same bit for bit.
+#pragma once
+
+#include <type_traits>
+
+#include "af_step.cuh"
+
+namespace af {
+
+struct ResidentParams {
+  const int* row_off;       // special cells by row (CSR over rows, sorted by column)
+  const SpecCell* row_spec;
+  uint4* halo;              // [2][blocks][2][W][halo_words]
+  void* slot;               // [2][to][from] Hmax words, see post_max
+  double* part;             // [2][blocks][2] volume and area at mass-report steps
+  unsigned* tag;            // first unused tag
+  int nr_max;               // rows of the tallest band
+  int gy;                   // row groups a band is cut into (at most 32 rows each)
+  double t_stop;
+  long long max_steps;
+};
+
+template <typename T>
+struct ResidentShape;
+template <>
+struct ResidentShape<float> {
+  static constexpr int threads = 512;
+  static constexpr int halo_words = 1;  // uint4 per column: {H, tag, Qx, tag}
+};
+template <>
+struct ResidentShape<double> {
+  static constexpr int threads = 512;
+  static constexpr int halo_words = 2;  // {H lo, tag, H hi, tag}, the same of Qx
+};
+
+// Dynamic shared memory of a band of nr rows of nx cells: two copies of H and
+// of Qx and one of Z over nr + 2 rows, two of Qy over nr + 1, per 32 cells the
+// special cells' mask and first entry, and the list of marches (gy row groups
+// per strip).
+template <typename T>
+__host__ __device__ inline size_t resident_smem(int nx, int nr, int gy) {
+  const size_t W = (size_t)nx + 1, nsx = (nx + 31) / 32;
+  return (W * (size_t)(7 * nr + 12) + 4) * sizeof(T) + 16 + nsx * (16 * (size_t)gy + 8 * (size_t)nr);
+}
+
+// Row groups of a band for `warps` warps: every group costs its rows and about
+// one and a half more (its first loads and the faces above and beside it).
+inline int resident_groups(int nx, int nr, int warps) {
+  const int nsx = (nx + 31) / 32;
+  int best = 1;
+  double cost = 1e300;
+  for (int g = 1; g <= nr; g++) {
+    const int rows = (nr + g - 1) / g;
+    if (rows > 32) continue;
+    const double c = (double)((nsx * g + warps - 1) / warps) * (rows + 1.5);
+    if (c < cost) {
+      cost = c;
+      best = g;
+    }
+  }
+  return best;
+}
+
+__device__ inline uint4 ld_relaxed(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ inline void st_relaxed(uint4* p, uint4 v) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y),
+               "r"(v.z), "r"(v.w)
+               : "memory");
+}
+
+__device__ inline void halo_put(uint4* at, float h, float q, unsigned tag) {
+  st_relaxed(at, make_uint4(__float_as_uint(h), tag, __float_as_uint(q), tag));
+}
+__device__ inline void halo_put(uint4* at, double h, double q, unsigned tag) {
+  st_relaxed(at, make_uint4((unsigned)__double2loint(h), tag, (unsigned)__double2hiint(h), tag));
+  st_relaxed(at + 1, make_uint4((unsigned)__double2loint(q), tag, (unsigned)__double2hiint(q), tag));
+}
+__device__ inline bool halo_get(const uint4* at, float& h, float& q, unsigned tag) {
+  const uint4 v = ld_relaxed(at);
+  h = __uint_as_float(v.x);
+  q = __uint_as_float(v.z);
+  return (v.y == tag) & (v.w == tag);
+}
+__device__ inline bool halo_get(const uint4* at, double& h, double& q, unsigned tag) {
+  const uint4 v = ld_relaxed(at), w = ld_relaxed(at + 1);
+  h = __hiloint2double((int)v.z, (int)v.x);
+  q = __hiloint2double((int)w.z, (int)w.x);
+  return (v.y == tag) & (v.w == tag) & (w.y == tag) & (w.w == tag);
+}
+
+// Two faces by the interior law; face k lies between cells (z0k, h0k) and
+// (z1k, h1k).  Discharges are the stored ones (FP64 forms Qold here).
+template <typename T>
+struct FaceIn {
+  T z0, h0, z1, h1, q0, qa, qb, qc, qd;
+};
+__device__ __forceinline__ void two_faces(const FaceIn<float>& a, const FaceIn<float>& b,
+                                          float /*dxinv*/, bool ea, bool eb,
+                                          const Phys<float>& ph, float& qa, float& qb) {
+  bool any = false;
+  const float2 q = flux2<true>(f2(a.z0, b.z0), f2(a.h0, b.h0), f2(a.z1, b.z1), f2(a.h1, b.h1),
+                               f2(a.q0, b.q0), f2(a.qa, b.qa), f2(a.qb, b.qb), f2(a.qc, b.qc),
+                               f2(a.qd, b.qd), true, ph, any);
+  qa = ea ? q.x : 0.0f;
+  qb = eb ? q.y : 0.0f;
+}
+__device__ __forceinline__ void two_faces(const FaceIn<double>& a, const FaceIn<double>& b,
+                                          double dxinv, bool ea, bool eb, const Phys<double>& ph,
+                                          double& qa, double& qb) {
+  const double ya0 = a.z0 + a.h0, ya1 = a.z1 + a.h1, yb0 = b.z0 + b.h0, yb1 = b.z1 + b.h1;
+  const double ha = gminT(gmaxT(ya0, ya1) - gmaxT(a.z0, a.z1), ph.max_hflow);
+  const double hb = gminT(gmaxT(yb0, yb1) - gmaxT(b.z0, b.z1), ph.max_hflow);
+  const bool wa = ea & (a.z0 != ph.nodata) & (a.z1 != ph.nodata) & (ha > ph.depth_thresh);
+  const bool wb = eb & (b.z0 != ph.nodata) & (b.z1 != ph.nodata) & (hb > ph.depth_thresh);
+  qa = 0.0;
+  qb = 0.0;
+  if (!__any_sync(0xffffffffu, wa | wb | !ph.fast)) return;
+  const double a0 = a.q0 * dxinv, aa = a.qa * dxinv, ab = a.qb * dxinv, ac = a.qc * dxinv,
+               ad = a.qd * dxinv;
+  const double b0 = b.q0 * dxinv, ba = b.qa * dxinv, bb = b.qb * dxinv, bc = b.qc * dxinv,
+               bd = b.qd * dxinv;
+  const double ma = (aa + ab + ac + ad) / 4.0, mb = (ba + bb + bc + bd) / 4.0;
+  bool xa, xb;
+  const double fa =
+      face_fast(ya0 - ya1, ha, a0 * a0 + ma * ma, a0, ph.dx, ph.rh, ph.rl, ph.gdt, ph.fn, xa);
+  const double fb =
+      face_fast(yb0 - yb1, hb, b0 * b0 + mb * mb, b0, ph.dx, ph.rh, ph.rl, ph.gdt, ph.fn, xb);
+  qa = wa ? fa : 0.0;
+  qb = wb ? fb : 0.0;
+  if (__any_sync(0xffffffffu, (xa & wa) | (xb & wb) | !ph.fast)) {
+    qa = face_any64(a.z0, a.h0, a.z1, a.h1, a0, aa, ab, ac, ad, ea, ph.fast, ph.dx, ph.rh, ph.rl,
+                    ph.gdt, ph.fn, ph.depth_thresh, ph.max_hflow, ph.nodata);
+    qb = face_any64(b.z0, b.h0, b.z1, b.h1, b0, ba, bb, bc, bd, eb, ph.fast, ph.dx, ph.rh, ph.rl,
+                    ph.gdt, ph.fn, ph.depth_thresh, ph.max_hflow, ph.nodata);
+  }
+}
+
+// Edge faces, out of line (a few lanes a step).
+static __device__ __noinline__ float edge_out(float h, float z, float sign, float g, float dx,
+                                              float nodata) {
+  return out_free(h, z, sign, g, dx, nodata);
+}
+static __device__ __noinline__ float edge_west(float h0, float z0, float h1, float z1, float g,
+                                               float dx, float nodata) {
+  return west_free(h0, z0, h1, z1, g, dx, nodata);
+}
+__device__ inline double edge_out(double h, double z, double sign, double g, double dx,
+                                  double nodata) {
+  return out_free64(h, z, sign, g, dx, nodata);
+}
+__device__ inline double edge_west(double h0, double z0, double h1, double z1, double g, double dx,
+                                   double nodata) {
+  return west_free64(h0, z0, h1, z1, g, dx, nodata);
+}
+
+// Special cells.  What their sources and boundaries are worth at a step's time
+// is worked out while the blocks exchange (the time is known then, dt is not
+// yet) and kept in shared memory, for bands of up to these many of each; in
+// the march it would hold up the band, and with it every other, by the few
+// thousand cycles of a hydrograph's look-up.  Larger bands look up as they go.
+constexpr int kBandSpecials = 128;
+constexpr int kBandSources = 256;
+
+// interpolate_bc_value of source s / boundary q at t (see apply_sources and
+// bc_depth).
+static __device__ __noinline__ double source_value(const StepParams& p, int s, double t) {
+  if (p.src_type[s] == AF_BC_QFIX) return p.src_value[s];
+  const int o = p.src_off[s];
+  return interp_series(p.src_times + o, p.src_vals + o, p.src_off[s + 1] - o, p.src_value[s], t,
+                       p.src_sorted[s] != 0);
+}
+template <typename T>
+static __device__ __noinline__ T boundary_depth(const StepParams& p, int q, double t) {
+  return bc_depth<T>(q,
+                     SeriesTable{p.bc_type, p.bc_value, p.bc_off, p.bc_times, p.bc_vals,
+                                 p.bc_sorted},
+                     t);
+}
+// One source's volume into a cell (apply_sources, src/main.cpp:253-259).
+template <typename T>
+__device__ inline T add_source(T h, double v, double dx, double dA, double dt) {
+  const double ps = v * dx * dt / dA;
+  h = h + T(ps);
+  if (h < T(0)) h = T(0);
+  return h;
+}
+// The segment k of the rain series that interp_series interpolates in at t
+// (times[k] <= t < times[k + 1], t inside the series), or -1.
+static __device__ __noinline__ int rain_segment(const StepParams& p, double t) {
+  const double* times = p.rain_times;
+  const int n = p.n_rain;
+  if (!p.rain_sorted || n < 2 || !(t > times[0] && t < times[n - 1])) return -1;
+  int lo = 0, hi = n - 1;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (times[mid] <= t) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Largest of a warp's ordered 64-bit images (ord_encode).
+__device__ __forceinline__ unsigned long long warp_max_ord(unsigned long long v) {
+  const unsigned hi = (unsigned)(v >> 32);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)v : 0u);
+  return ((unsigned long long)mh << 32) | ml;
+}
+
+__device__ inline float cell_update(float h, float qw, float qe, float qn, float qs, bool rain,
+                                    const StepScal<float>& sc) {
+  // The operations of update_cells<float>, one cell in a pair.
+  const float2 a = __ffma2_rn(f2(qe, qs), f2(-1.0f, -1.0f), f2(qw, qn));
+  const float2 d = __fadd2_rn(f2(a.x, 0.0f), f2(a.y, 0.0f));
+  const float2 inc = __ffma2_rn(f2(sc.dt_dA, 0.0f), d, f2(rain ? sc.rain_depth : 0.0f, 0.0f));
+  return fmaxf(__fadd2_rn(f2(h, 0.0f), inc).x, 0.0f);
+}
+__device__ inline double cell_update(double h, double qw, double qe, double qn, double qs,
+                                     bool rain, const StepScal<double>& sc) {
+  return update_cell(h, qw, qe, qn, qs, rain, sc.rain_depth, sc.dtT, sc.dAT, sc.ph);
+}
+
+// Hmax of all blocks: each writes its own (the depth's ordered image with the
+// step's tag beside every 4 bytes) into every block's row and polls only its
+// own row, one warp per block.  Cycles per exchange of 148 blocks by itself:
+// 2900 with 8-byte words (FP32), 3700 with 16-byte words (FP64); all polling
+// one shared row 5800, two rounds in groups of 13 4100; an atomic maximum with
+// a counted arrival 3000, but 5000 in the loop, where its release also waits
+// for the halo stores.
+__device__ inline unsigned ord32(float x) {
+  const unsigned u = __float_as_uint(x);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ inline float ord32_value(unsigned u) {
+  return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
+}
+struct MaxF32 {
+  using Bits = unsigned;
+  using Word = uint2;
+  __device__ static Bits of(float m) { return ord32(m); }
+  __device__ static double value(Bits b) { return (double)ord32_value(b); }
+  __device__ static Bits warp(Bits b) { return __reduce_max_sync(0xffffffffu, b); }
+  __device__ static void put(Word* p, Bits b, unsigned tag) {
+    asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(b), "r"(tag)
+                 : "memory");
+  }
+  __device__ static bool get(const Word* p, Bits& b, unsigned tag) {
+    unsigned t;
+    asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(b), "=r"(t) : "l"(p)
+                 : "memory");
+    return t == tag;
+  }
+};
+struct MaxF64 {
+  using Bits = unsigned long long;
+  using Word = uint4;
+  __device__ static Bits of(double m) { return ord_encode(m); }
+  __device__ static double value(Bits b) { return ord_decode(b); }
+  __device__ static Bits warp(Bits b) { return warp_max_ord(b); }
+  __device__ static void put(Word* p, Bits b, unsigned tag) {
+    st_relaxed(p, make_uint4((unsigned)b, tag, (unsigned)(b >> 32), tag));
+  }
+  __device__ static bool get(const Word* p, Bits& b, unsigned tag) {
+    const uint4 x = ld_relaxed(p);
+    b = ((Bits)x.z << 32) | x.x;
+    return (x.y == tag) & (x.w == tag);
+  }
+};
+template <typename T>
+using MaxOf = typename std::conditional<sizeof(T) == 8, MaxF64, MaxF32>::type;
+
+template <typename M>
+__device__ __forceinline__ void post_max(void* slot, int nb, int buf, int b, unsigned tag,
+                                         typename M::Bits v) {
+  typename M::Word* const to = static_cast<typename M::Word*>(slot) + (size_t)buf * nb * nb + b;
+  for (int k = threadIdx.x & 31; k < nb; k += 32) M::put(to + (size_t)k * nb, v, tag);
+}
+// False when a wait ran out.
+template <typename M>
+__device__ __forceinline__ bool collect_max(void* slot, int nb, int buf, int b, unsigned tag,
+                                            typename M::Bits& v) {
+  constexpr int K = 5;  // loads in flight per lane: one round on up to 160 blocks
+  const typename M::Word* const row =
+      static_cast<const typename M::Word*>(slot) + ((size_t)buf * nb + b) * nb;
+  const int lane = threadIdx.x & 31;
+  typename M::Bits m = 0;
+  bool ok = true;
+  for (int k0 = lane; k0 - lane < nb; k0 += 32 * K) {
+    typename M::Bits x[K];
+    bool all = false;
+    for (int w = 0; w < (int)kRingWaitLimit && !all; w++) {
+      all = true;
+#pragma unroll
+      for (int u = 0; u < K; u++) all &= M::get(row + min(k0 + 32 * u, nb - 1), x[u], tag);
+    }
+    ok &= all;
+#pragma unroll
+    for (int u = 0; u < K; u++) m = x[u] > m ? x[u] : m;
+  }
+  v = M::warp(m);
+  return __all_sync(0xffffffffu, ok);
+}
+
+// A special cell's new depth: its sources, the update, its boundary depth.  `e`
+// is its entry; src (by source) and bc its band's values, or null.
+template <typename T>
+static __device__ __noinline__ T special_cell(const StepParams& p, const StepScal<T>& sc,
+                                              const SpecCell* e, const double* src, const T* bc,
+                                              T h, T qw, T qe, T qn, T qs, bool rain) {
+  for (int s = e->s0; s < e->s1; s++)
+    h = add_source(h, src ? src[s] : source_value(p, s, sc.t), p.dx, p.dA, sc.dt);
+  h = cell_update(h, qw, qe, qn, qs, rain, sc);
+  if (e->bc >= 0) h = bc ? *bc : boundary_depth<T>(p, e->bc, sc.t);
+  return h;
+}
+
+// What warp 0 carries from step to step, in shared memory so that it takes no
+// registers of the march.
+struct Clock {
+  double t, dt_last, hmax, rate, next_mass;
+  double r_t0, r_t1, r_v0, r_v1;  // the rain series' segment of the last look-up
+  int status, mass_count;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
+    k_resident(const __grid_constant__ StepParams p, const __grid_constant__ ResidentParams rp) {
+  constexpr int NT = ResidentShape<T>::threads, NW = NT / 32;
+  constexpr int HW = ResidentShape<T>::halo_words;
+  extern __shared__ __align__(16) unsigned char s_mem[];
+  __shared__ StepScal<T> s_sc;
+  using M = MaxOf<T>;
+  __shared__ typename M::Bits s_max[NW];
+  __shared__ double s_v[NW], s_a[NW];
+  __shared__ int s_done, s_fail, s_nseg;
+  __shared__ double s_src[kBandSources];  // the band's sources' values at the step's time
+  __shared__ T s_bc[kBandSpecials];       // and its special cells' boundary depths
+  __shared__ SpecCell s_spec[kBandSpecials];
+  __shared__ Clock s_clock;
+  SimCtl* ctl = p.ctl;
+  int lane;  // read once: not recomputed from the thread index in the loop
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int nb = gridDim.x, b = blockIdx.x;
+  const int nx = p.nx, ny = p.ny, P = p.P, W = nx + 1;
+  // Band of rows: the first ny % nb bands have one row more.
+  const int base = ny / nb, more = ny % nb;
+  const int r0 = b * base + min(b, more);
+  const int nr = base + (b < more ? 1 : 0);
+  // Local row l of H, Z and Qx is grid row r0 - 1 + l, of Qy the faces north
+  // of grid row r0 + l.  A row's last column (nx) is H's, Z's and Qy's next
+  // row's left neighbour of column 0, never used.
+  const int nH = (rp.nr_max + 2) * W, nY = (rp.nr_max + 1) * W;
+  T* const H0 = reinterpret_cast<T*>(s_mem) + 1;
+  T* const Z = H0 + 2 * nH;
+  T* const X0 = Z + nH;
+  T* const Y0 = X0 + 2 * nH + 1;
+  const int nsx = (nx + 31) / 32;
+  int4* const segs = reinterpret_cast<int4*>(
+      s_mem + ((((size_t)W * (7 * rp.nr_max + 12) + 4) * sizeof(T) + 15) & ~(size_t)15));
+  uint2* const at32 = reinterpret_cast<uint2*>(segs + nsx * rp.gy);  // {mask, first entry}
+
+  // ---- the loop's start: time, Hmax and limits, the same in every block
+  const double t_start = ctl->t;
+  const int par0 = ctl->parity;
+  const unsigned tag0 = *rp.tag;
+  long long n = 0;  // steps of this launch
+  const bool go = ctl->status == 0 && t_start < rp.t_stop && rp.max_steps > 0;
+  if (tid == 0) {
+    Clock& k = s_clock;
+    k.t = t_start;
+    k.dt_last = ctl->dt_last;
+    k.hmax = ctl->hmax;
+    k.rate = ctl->rain_rate;
+    k.next_mass = ctl->next_mass;
+    k.r_t0 = k.r_v0 = k.r_v1 = 0.0;
+    k.r_t1 = -1.0;
+    k.status = ctl->status;
+    k.mass_count = ctl->mass_count;
+    fill_scalars(p, k.t, step_dt(p, k.hmax), k.rate, k.next_mass, par0, s_sc);
+    s_fail = 0;
+    // The band's marches: strip, first and last row.
+    int q = 0;
+    for (int gi = 0; gi < rp.gy; gi++) {
+      const int ra = nr * gi / rp.gy, rb = nr * (gi + 1) / rp.gy;
+      for (int x = 0; x < nsx && ra < rb; x++) segs[q++] = make_int4(x, ra, rb, 0);
+    }
+    s_nseg = q;
+  }
+  // The band's special cells and (consecutive, as cells are) their sources.
+  const int e0 = rp.row_off[r0], ne = rp.row_off[r0 + nr] - e0;
+  const int src0 = ne > 0 ? rp.row_spec[e0].s0 : 0;
+  const int nsrc = ne > 0 ? rp.row_spec[e0 + ne - 1].s1 - src0 : 0;
+  const bool cached = ne <= kBandSpecials && nsrc <= kBandSources;
+  auto band_values = [&](double at) {
+    for (int k = tid; k < nsrc; k += NT) s_src[k] = source_value(p, src0 + k, at);
+    for (int e = tid; e < ne; e += NT) {
+      const int q = rp.row_spec[e0 + e].bc;
+      if (q >= 0) s_bc[e] = boundary_depth<T>(p, q, at);
+    }
+  };
+  if (go) {
+    const T* gH = static_cast<const T*>(p.H[par0]);
+    const T* gZ = static_cast<const T*>(p.DEM);
+    const T* gX = static_cast<const T*>(p.Qx[par0]);
+    const T* gY = static_cast<const T*>(p.Qy[par0]);
+    for (int l = warp; l < nr + 2; l += NW) {
+      const int r = r0 - 1 + l;
+      const bool in = r >= 0 && r < ny;
+      for (int i = lane - 1; i <= nx; i += 32) {
+        const long long g = (long long)r * P + i;
+        const bool cell = in && i >= 0 && i < nx;
+        if (i < nx) {
+          H0[l * W + i] = cell ? gH[g] : T(0);
+          H0[nH + l * W + i] = T(0);
+          Z[l * W + i] = cell ? gZ[g] : T(0);
+        }
+        if (i >= 0) {
+          X0[l * W + i] = in ? gX[g] : T(0);
+          X0[nH + l * W + i] = T(0);
+        }
+        if (l <= nr && i < nx) {
+          Y0[l * W + i] = i >= 0 ? gY[g + P] : T(0);
+          Y0[nY + l * W + i] = T(0);
+        }
+      }
+    }
+    for (int k = tid; k < nr * nsx; k += NT) {
+      const int r = r0 + k / nsx, c0 = k % nsx * 32;
+      int lo = rp.row_off[r], hi = rp.row_off[r + 1];  // first entry at or past column c0
+      const int end = hi;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rp.row_spec[mid].col < c0) lo = mid + 1;
+        else hi = mid;
+      }
+      unsigned m = 0u;
+      for (int e = lo; e < end && rp.row_spec[e].col < c0 + 32; e++)
+        m |= 1u << (rp.row_spec[e].col - c0);
+      at32[k] = make_uint2(m, (unsigned)lo);
+    }
+    if (cached) {
+      for (int e = tid; e < ne; e += NT) s_spec[e] = rp.row_spec[e0 + e];
+      band_values(t_start);
+    }
+  }
+  __syncthreads();
+
+  const int nseg = s_nseg;
+  bool failed = false;
+#pragma unroll 1
+  while (go) {
+    const unsigned tag = tag0 + (unsigned)n;
+    const int buf = (int)(n & 1);
+    const StepScal<T>& sc = s_sc;  // rewritten by the last warp once nobody needs it
+    const T* const H = H0 + buf * nH;
+    T* const Hn = H0 + (buf ^ 1) * nH;
+    const T* const X = X0 + buf * nH;
+    T* const Xn = X0 + (buf ^ 1) * nH;
+    const T* const Y = Y0 + buf * nY;
+    T* const Yn = Y0 + (buf ^ 1) * nY;
+    const Phys<T> ph = sc.ph;
+    const T dxinv = sc.dxinvT;
+    const bool mass = sc.mass, rain_on = sc.rain_on;
+    uint4* const my_halo = rp.halo + ((size_t)(buf * nb + b) * 2) * W * HW;
+    T m = T(-FLT_MAX);
+    double v = 0.0, a = 0.0;
+#pragma unroll 1
+    for (int seg = warp; seg < nseg; seg += NW) {
+      const int4 sg = segs[seg];
+      const int sx = sg.x, ra = sg.y, rb = sg.z;
+      const int c = sx * 32 + lane;
+      const int cc = min(c, nx - 1);
+      const bool own = c < nx, east = c == nx - 1;
+      // Faces above row ra (their own columns), and on the strip's east side
+      // of row ra + lane.
+      int k = (ra + 1) * W + cc, g = ra * W + cc;
+      T h = H[k], z = Z[k], x0 = X[k], x1 = X[k + 1], y0 = Y[g];
+      T qn, qE;
+      {
+        const int ce = min(sx * 32 + 32, nx - 1);
+        const int re = min(ra + lane, rb - 1);
+        const int ke = (re + 1) * W + ce, ge = re * W + ce;
+        two_faces(FaceIn<T>{Z[ke - 1], H[ke - 1], Z[ke], H[ke], X[ke], Y[ge - 1], Y[ge],
+                            Y[ge + W - 1], Y[ge + W]},
+                  FaceIn<T>{Z[k - W], H[k - W], z, h, y0, X[k - W], X[k + 1 - W], x0, x1}, dxinv,
+                  sx < nsx - 1, r0 + ra > 0, ph, qE, qn);
+      }
+      if (r0 + ra == 0) qn = p.nf ? edge_out(h, z, T(-1), ph.g, ph.dx, ph.nodata) : T(0);
+      if (ra == 0 && own) Yn[g] = qn;  // further down the group above stores it
+      T hW = H[k - 1], zW = Z[k - 1], yW = Y[g - 1];
+      const bool full = sx > 0 && sx < nsx - 1;  // no edge column, every lane owns a cell
+#pragma unroll 1
+      for (int r = ra; r < rb; r++) {
+        const T hN = H[k + W], zN = Z[k + W], x0N = X[k + W], x1N = X[k + W + 1];
+        const T hNW = H[k + W - 1], zNW = Z[k + W - 1];
+        const T s0 = Y[g + W], sW = Y[g + W - 1];
+        const unsigned specials = at32[r * nsx + sx].x;
+        const bool south = r0 + r + 1 < ny;
+        T qw, qs;
+        two_faces(FaceIn<T>{zW, hW, z, h, x0, yW, y0, sW, s0},
+                  FaceIn<T>{z, h, zN, hN, s0, x0, x1, x0N, x1N}, dxinv, true, south, ph, qw, qs);
+        T qe = __shfl_down_sync(0xffffffffu, qw, 1);
+        const T qEr = __shfl_sync(0xffffffffu, qE, r - ra);
+        if (lane == 31) qe = qEr;
+        const bool valid = z != ph.nodata;
+        T hn;
+        if (full & south & (specials == 0u)) {
+          hn = cell_update(h, qw, qe, qn, qs, rain_on && valid, sc);
+        } else {
+          if (!south) qs = p.sf ? edge_out(h, z, T(1), ph.g, ph.dx, ph.nodata) : T(0);
+          if (sx == 0) {
+            if (lane == 0)
+              qw = p.wf ? edge_west(h, z, H[k + 1], Z[k + 1], ph.g, ph.dx, ph.nodata) : T(0);
+          }
+          if (east) {
+            qe = p.ef ? edge_out(h, z, T(1), ph.g, ph.dx, ph.nodata) : T(0);
+            Xn[k + 1] = qe;
+            if ((r == 0) & (b > 0)) halo_put(my_halo + (size_t)nx * HW, T(0), qe, tag);
+            if ((r == nr - 1) & (b < nb - 1))
+              halo_put(my_halo + (size_t)(W + nx) * HW, T(0), qe, tag);
+          }
+          hn = cell_update(h, qw, qe, qn, qs, rain_on && valid, sc);
+          if ((specials >> lane) & 1u) {
+            const int e = (int)at32[r * nsx + sx].y + __popc(specials & ((1u << lane) - 1u));
+            hn = cached ? special_cell<T>(p, sc, &s_spec[e - e0], s_src - src0, &s_bc[e - e0], h, qw,
+                                          qe, qn, qs, rain_on && valid)
+                        : special_cell<T>(p, sc, &rp.row_spec[e], nullptr, nullptr, h, qw, qe, qn,
+                                          qs, rain_on && valid);
+          }
+        }
+        if (own) {
+          Hn[k] = hn;
+          Xn[k] = qw;
+          Yn[g + W] = qs;
+          if (valid) m = hn > m ? hn : m;  // a NaN never wins
+        }
+        if ((r == 0) | (r == nr - 1) | mass) {
+          if (own) {
+            if ((r == 0) & (b > 0)) halo_put(my_halo + (size_t)c * HW, hn, qw, tag);
+            if ((r == nr - 1) & (b < nb - 1))
+              halo_put(my_halo + (size_t)(W + c) * HW, hn, qw, tag);
+            if (mass) {
+              const double hv = (double)hn;
+              v += hv * p.dA;
+              if (hv > 0.01) a += p.dA;
+            }
+          }
+        }
+        k += W;
+        g += W;
+        h = hN;
+        z = zN;
+        hW = hNW;
+        zW = zNW;
+        x0 = x0N;
+        x1 = x1N;
+        y0 = s0;
+        yW = sW;
+        qn = qs;
+      }
+    }
+    const typename M::Bits mo = M::warp(M::of(m));
+    if (mass) {
+      v = warp_sum(v);
+      a = warp_sum(a);
+    }
+    if (lane == 0) {
+      s_max[warp] = mo;
+      s_v[warp] = v;
+      s_a[warp] = a;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      // ---- Hmax of all blocks, then the next step's time, dt and constants
+      const typename M::Bits bm = M::warp(lane < NW ? s_max[lane] : 0);
+      if (mass) {
+        if (lane == 0) {
+          double sv = 0.0, sa = 0.0;
+          for (int w = 0; w < NW; w++) {
+            sv += s_v[w];
+            sa += s_a[w];
+          }
+          rp.part[(size_t)(buf * nb + b) * 2] = sv;
+          rp.part[(size_t)(buf * nb + b) * 2 + 1] = sa;
+          __threadfence();
+        }
+        __syncwarp();
+      }
+      post_max<M>(rp.slot, nb, buf, b, tag, bm);
+      // Time and rain rate while the others' Hmax is on its way.
+      Clock& ck = s_clock;
+      const double t = sc.t + sc.dt;
+      double rate = 0.0;
+      if (p.n_rain > 0) {
+        const double t0 = ck.r_t0, t1 = ck.r_t1;
+        if (t0 <= t && t < t1) {  // still in the segment: interp_series' own expression
+          const double v0 = ck.r_v0;
+          rate = v0 + (t - t0) / (t1 - t0) * (ck.r_v1 - v0);
+        } else {
+          const int k = rain_segment(p, t);
+          rate = interp_series(p.rain_times, p.rain_rates, p.n_rain, 0.0, t, p.rain_sorted != 0);
+          __syncwarp();
+          if (lane == 0) {
+            ck.r_t1 = -1.0;
+            if (k >= 0) {
+              ck.r_t0 = p.rain_times[k];
+              ck.r_t1 = p.rain_times[k + 1];
+              ck.r_v0 = p.rain_rates[k];
+              ck.r_v1 = p.rain_rates[k + 1];
+            }
+          }
+        }
+      }
+      typename M::Bits gm;
+      const bool ok = collect_max<M>(rp.slot, nb, buf, b, tag, gm);
+      const double gd = M::value(gm);
+      // The bookkeeping of fold_step, in every block alike.
+      const double hmax = gd > -(double)FLT_MAX ? gd : -DBL_MAX;
+      double next_mass = ck.next_mass;
+      int mass_count = ck.mass_count;
+      if (mass) {
+        if (b == 0 && mass_count < ctl->mass_cap) {
+          __threadfence();
+          const double* part = rp.part + (size_t)buf * nb * 2;
+          double s = 0.0, cs = 0.0, ar = 0.0;
+          for (int k = lane; k < nb; k += 32) {
+            kahan_add(s, cs, __ldcg(&part[2 * k]));
+            ar += __ldcg(&part[2 * k + 1]);
+          }
+          double S = 0.0, C = 0.0, A = 0.0;
+          for (int l = 0; l < 32; l++) {
+            kahan_add(S, C, __shfl_sync(0xffffffffu, s, l));
+            C += __shfl_sync(0xffffffffu, cs, l);
+            A += __shfl_sync(0xffffffffu, ar, l);
+          }
+          if (lane == 0) {
+            p.mass_series[3 * mass_count] = t;
+            p.mass_series[3 * mass_count + 1] = S + C;
+            p.mass_series[3 * mass_count + 2] = A;
+          }
+          mass_count++;
+        }
+        next_mass += p.mass_int;
+      }
+      const double dt_last = sc.dt;
+      const bool bad = !(dt_last > 0.0) || !(t < 1.0e300) || !(hmax == hmax);
+      const int status = !ok ? 2 : bad ? 1 : 0;
+      const bool done = status != 0 || !(t < rp.t_stop) || n + 1 >= rp.max_steps;
+      __syncwarp();
+      if (lane == 0) {
+        if (!done) {
+          // The fields of fill_scalars that change from step to step.
+          const double dt = step_dt(p, hmax);
+          s_sc.t = t;
+          s_sc.dt = dt;
+          s_sc.mass = p.mass_int > 0.0 && (t + dt >= next_mass);
+          s_sc.rain_on = rate > 0.0;
+          s_sc.rain_depth = T(rate * dt);
+          s_sc.dtT = T(dt);
+          s_sc.ph.gdt = T(p.g * dt);
+          if (sizeof(T) == 4) {
+            s_sc.dt_dA = T(dt / p.dA);
+            s_sc.ph.gdt_fn2 = T(p.g * dt * p.fpn * p.fpn * p.dxinv);
+          } else {
+            s_sc.ph.fast = face_range_ok(p.dx, p.fpn, p.depth_thresh, p.max_hflow, p.g * dt);
+          }
+        }
+        if (!ok) s_fail = 1;
+        s_done = done;
+        ck.t = t;
+        ck.dt_last = dt_last;
+        ck.hmax = hmax;
+        ck.rate = rate;
+        ck.next_mass = next_mass;
+        ck.status = status;
+        ck.mass_count = mass_count;
+      }
+    } else {
+      if (cached && ne > 0) {  // for the next step's time
+        const double at = sc.t + sc.dt;
+        for (int k = tid - 32; k < nsrc; k += NT - 32) s_src[k] = source_value(p, src0 + k, at);
+        for (int e = tid - 32; e < ne; e += NT - 32)
+          if (s_spec[e].bc >= 0) s_bc[e] = boundary_depth<T>(p, s_spec[e].bc, at);
+      }
+      // ---- the neighbours' rows
+      const uint4* const above = rp.halo + ((size_t)(buf * nb + b - 1) * 2 + 1) * W * HW;
+      const uint4* const below = rp.halo + ((size_t)(buf * nb + b + 1) * 2) * W * HW;
+      bool ok = true;
+      constexpr int K = 4;  // columns in flight per thread
+      for (int k0 = tid - 32; k0 < 2 * W; k0 += K * (NT - 32)) {
+        T hh[K], qq[K];
+        bool got[K], want[K];
+#pragma unroll
+        for (int u = 0; u < K; u++) {
+          const int k = k0 + u * (NT - 32);
+          want[u] = k < W ? b > 0 : (k < 2 * W && b < nb - 1);
+          got[u] = !want[u];
+          hh[u] = qq[u] = T(0);
+        }
+        for (int w = 0; w < (int)kRingWaitLimit && !(got[0] & got[1] & got[2] & got[3]); w++) {
+#pragma unroll
+          for (int u = 0; u < K; u++) {
+            const int k = k0 + u * (NT - 32);
+            if (!got[u])
+              got[u] = halo_get(k < W ? above + (size_t)k * HW : below + (size_t)(k - W) * HW,
+                                hh[u], qq[u], tag);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < K; u++) {
+          const int k = k0 + u * (NT - 32);
+          ok &= got[u];
+          if (want[u]) {
+            const int l = k < W ? 0 : nr + 1, i = k < W ? k : k - W;
+            if (i < nx) Hn[l * W + i] = hh[u];
+            Xn[l * W + i] = qq[u];
+          }
+        }
+      }
+      if (!ok) s_fail = 1;
+    }
+    __syncthreads();
+    n++;
+    if (s_fail) {
+      failed = true;
+      break;
+    }
+    if (s_done) break;
+  }
+
+  // ---- the state back to its planes, and the control block
+  if (failed && tid == 0) atomicExch(&ctl->status, 2);
+  const int par = (par0 + (int)(n & 1)) & 1;
+  if (!failed && n > 0) {
+    const int buf = (int)(n & 1);
+    T* gH = static_cast<T*>(p.H[par]);
+    T* gX = static_cast<T*>(p.Qx[par]);
+    T* gY = static_cast<T*>(p.Qy[par]);
+    for (int l = warp; l < nr + (b == nb - 1 ? 1 : 0); l += NW) {
+      const long long g = (long long)(r0 + l) * P;
+      for (int i = lane; i <= nx; i += 32) {
+        if (l < nr) {
+          if (i < nx) gH[g + i] = H0[buf * nH + (l + 1) * W + i];
+          gX[g + i] = X0[buf * nH + (l + 1) * W + i];
+        }
+        if (i < nx) gY[g + i] = Y0[buf * nY + l * W + i];
+      }
+    }
+  }
+  if (b == 0 && tid == 0) {
+    const long long limit = 0x3FFFFFFFFFFFFFFFLL;
+    ctl->t_stop = rp.t_stop;
+    ctl->step_stop = rp.max_steps > limit - ctl->step ? limit : ctl->step + rp.max_steps;
+    ctl->step += n;
+    ctl->done = 1;
+    ctl->arrive = 0u;
+    if (n > 0) {
+      const Clock& k = s_clock;
+      ctl->t = k.t;
+      ctl->hmax = k.hmax;
+      ctl->dt_last = k.dt_last;
+      ctl->rain_rate = k.rate;
+      ctl->next_mass = k.next_mass;
+      ctl->mass_count = k.mass_count;
+      ctl->parity = par;
+      if (k.status != 0) atomicMax(&ctl->status, k.status);
+      *rp.tag = tag0 + (unsigned)n + 16u;
+    }
+  }
+}
+
+}  // namespace af

@@ -17,6 +17,7 @@
 #include <sys/stat.h>
 
 #include "af_output.h"
+#include "af_resident.cuh"
 #include "af_simcore.cuh"
 #include "af_xfer.h"
 
@@ -249,6 +250,12 @@ struct Sim {
   DevBuf bc_type, bc_value, bc_off, bc_times, bc_vals, bc_sorted;
   DevBuf rain_times, rain_rates, spec_off, spec;
   DevBuf ctl, partials, mass_series;
+  bool resident = false;  // small grid: the whole loop in one launch (af_resident.cuh)
+  DevBuf row_off, row_spec, halo, slot, rpart, rtag;
+  size_t halo_bytes = 0, slot_bytes = 0;
+  ResidentParams rprm{};
+  unsigned rblocks = 0;
+  size_t rsmem = 0;
   SimCtl* pinned_ctl = nullptr;
   StepParams prm{};
   dim3 grid, block;
@@ -351,6 +358,50 @@ static int pick_shape(Sim& s) {
   s.grid = dim3((unsigned)(tiles < slots ? tiles : slots));
   s.block = dim3(32 * s.WY);
   return AF_OK;
+}
+
+// Whether the grid's state fits on chip, and the resident loop's bands.  The
+// strip kernels' switches (and host-driven launches) keep the strip kernels;
+// AF_SIM_RESIDENT=0/1 forces the choice where the state fits.
+static bool pick_resident(Sim& s) {
+  const char* force = getenv("AF_SIM_RESIDENT");
+  if (force && force[0] == '0') return false;
+  const char* direct = getenv("AF_SIM_DIRECT_LAUNCH");
+  if (direct && direct[0] && direct[0] != '0') return false;
+  if (!force && (getenv("AF_SIM_VARIANT") || getenv("AF_SIM_ROWS") || getenv("AF_SIM_TMA")))
+    return false;
+  int dev = 0, sms = 0, coop = 0, smem = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      !coop)
+    return false;
+  const bool f64 = s.prec == AF_PREC_F64;
+  const int nb = std::min(sms, s.c.ny);
+  const int nr = (s.c.ny + nb - 1) / nb;
+  const int threads = f64 ? ResidentShape<double>::threads : ResidentShape<float>::threads;
+  const int gy = resident_groups(s.c.nx, nr, threads / 32);
+  const size_t need =
+      f64 ? resident_smem<double>(s.c.nx, nr, gy) : resident_smem<float>(s.c.nx, nr, gy);
+  const void* fn = f64 ? resident_kernel_f64() : resident_kernel_f32();
+  cudaFuncAttributes a;
+  if (cudaFuncGetAttributes(&a, fn) != cudaSuccess || need + a.sharedSizeBytes > (size_t)smem)
+    return false;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem - (int)a.sharedSizeBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, need) != cudaSuccess ||
+      per_sm < 1)
+    return false;
+  s.rblocks = (unsigned)nb;
+  s.rsmem = need;
+  s.rprm.nr_max = nr;
+  s.rprm.gy = gy;
+  return true;
 }
 
 // The tensor map of the field planes (see encode_field_planes).
@@ -464,6 +515,46 @@ static int read_ctl(Sim& s) {
 
 static int write_ctl(Sim& s) {
   AF_CUDA(cudaMemcpyAsync(s.ctl.p, s.pinned_ctl, sizeof(SimCtl), cudaMemcpyHostToDevice, s.st));
+  AF_CUDA(cudaStreamSynchronize(s.st));
+  return AF_OK;
+}
+
+// The exchange of the resident loop as new: nothing posted, no tag used.
+static int reset_resident(Sim& s) {
+  AF_CUDA(cudaMemsetAsync(s.halo.p, 0, s.halo_bytes, s.st));
+  AF_CUDA(cudaMemsetAsync(s.slot.p, 0, s.slot_bytes, s.st));
+  static const unsigned first = 1u;  // 0 is never a step's tag
+  AF_CUDA(cudaMemcpyAsync(s.rprm.tag, &first, sizeof first, cudaMemcpyHostToDevice, s.st));
+  return AF_OK;
+}
+
+// The resident loop's workspaces and its special cells by row.
+static int setup_resident(Sim& s, std::vector<SpecCell> spec) {
+  std::sort(spec.begin(), spec.end(), [](const SpecCell& a, const SpecCell& b) {
+    return a.row != b.row ? a.row < b.row : a.col < b.col;
+  });
+  std::vector<int> off((size_t)s.c.ny + 1, 0);
+  for (const SpecCell& e : spec) off[e.row + 1]++;
+  for (int j = 0; j < s.c.ny; j++) off[j + 1] += off[j];
+  AF_TRY(upload(s.row_off, off, s.st));
+  AF_TRY(upload(s.row_spec, spec, s.st));
+  const size_t hw = s.prec == AF_PREC_F64 ? ResidentShape<double>::halo_words
+                                          : ResidentShape<float>::halo_words;
+  s.halo_bytes = (size_t)4 * s.rblocks * (s.c.nx + 1) * hw * sizeof(uint4);
+  AF_TRY(alloc_field(s.halo, s.halo_bytes, 1));
+  s.slot_bytes = (size_t)2 * s.rblocks * s.rblocks * sizeof(uint4);
+  AF_TRY(alloc_field(s.slot, s.slot_bytes, 1));
+  AF_TRY(alloc_field(s.rtag, 1, sizeof(unsigned)));
+  AF_TRY(alloc_field(s.rpart, (size_t)4 * s.rblocks, 8));
+  ResidentParams& r = s.rprm;
+  r.row_off = (const int*)s.row_off.p;
+  r.row_spec = (const SpecCell*)s.row_spec.p;
+  r.halo = (uint4*)s.halo.p;
+  r.part = (double*)s.rpart.p;
+  r.slot = s.slot.p;
+  r.tag = (unsigned*)s.rtag.p;
+  AF_TRY(reset_resident(s));
+  // Pageable sources: wait until the copies have left host memory.
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }
@@ -724,7 +815,9 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   p.partials = static_cast<double*>(s->partials.p);
   p.mass_series = static_cast<double*>(s->mass_series.p);
   p.use_cond = 0;
-  AF_TRY(build_graph(*s));
+  s->resident = pick_resident(*s);
+  if (s->resident) AF_TRY(setup_resident(*s, std::move(tb.spec)));
+  else AF_TRY(build_graph(*s));
   AF_CUDA(cudaStreamSynchronize(s->st));
   *out = s.release();
   return AF_OK;
@@ -733,6 +826,17 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
 static int launch(Sim& s, double t_stop, long long max_steps) {
   AF_CUDA(cudaSetDevice(s.device));
   SimCtl* ctl = static_cast<SimCtl*>(s.ctl.p);
+  if (s.resident) {
+    const bool f64 = s.prec == AF_PREC_F64;
+    s.rprm.t_stop = t_stop;
+    s.rprm.max_steps = max_steps;
+    void* args[] = {&s.prm, &s.rprm};
+    AF_CUDA(cudaLaunchCooperativeKernel(
+        f64 ? resident_kernel_f64() : resident_kernel_f32(), dim3(s.rblocks),
+        dim3(f64 ? ResidentShape<double>::threads : ResidentShape<float>::threads), args, s.rsmem,
+        s.st));
+    return AF_OK;
+  }
   if (s.use_cond) {
     int use = 1;
     void* bargs[] = {&ctl, &t_stop, &max_steps, &s.cond, &use};
@@ -1293,6 +1397,8 @@ static int restore(Sim& s, const char* path) {
   ctl.done = 1;
   ctl.status = 0;
   *s.pinned_ctl = ctl;
+  // A loop that gave up may have left its exchange half done.
+  if (s.resident) AF_TRY(reset_resident(s));
   return write_ctl(s);
 }
 

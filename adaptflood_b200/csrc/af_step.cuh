@@ -1842,6 +1842,8 @@ constexpr int kStepVariants = 5;
 constexpr StepVariant kStepVariant[kStepVariants] = {{1, 16}, {1, 12}, {1, 20}, {4, 4}, {2, 8}};
 const void* step_kernel_f64(int variant, bool tma = true);
 const void* step_kernel_f32(int variant, bool tma = true);
+const void* resident_kernel_f64();  // the resident loop (af_resident.cuh)
+const void* resident_kernel_f32();
 const void* batch_kernel_f64(int variant);
 const void* batch_kernel_f32(int variant);
 // Begin and fold kernels of the batch loop (one block of kFoldThreads),

@@ -1,6 +1,6 @@
 // af_step_f32.cu -- FP32 instantiation of the fused step (FP32 state and
 // arithmetic; FP64 time, dt, hydrograph interpolation and volume sums).
-#include "af_step.cuh"
+#include "af_resident.cuh"
 
 namespace af {
 // Indices follow kStepVariant in af_step.cuh.
@@ -31,6 +31,7 @@ const void* batch_kernel_f32(int variant) {
     default: return (const void*)&k_batch_step<float, 1, 16>;
   }
 }
+const void* resident_kernel_f32() { return (const void*)&k_resident<float>; }
 const void* batch_begin_f32() { return (const void*)&k_batch_begin<float>; }
 const void* batch_fold_f32() { return (const void*)&k_batch_fold<float>; }
 }  // namespace af

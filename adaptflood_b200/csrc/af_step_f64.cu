@@ -1,6 +1,6 @@
 // af_step_f64.cu -- FP64 instantiation of the fused step.  Compiled with
 // -fmad=false so each expression rounds as the reference's C++ does.
-#include "af_step.cuh"
+#include "af_resident.cuh"
 
 namespace af {
 // Indices follow kStepVariant in af_step.cuh.
@@ -31,6 +31,7 @@ const void* batch_kernel_f64(int variant) {
     default: return (const void*)&k_batch_step<double, 1, 16>;
   }
 }
+const void* resident_kernel_f64() { return (const void*)&k_resident<double>; }
 const void* batch_begin_f64() { return (const void*)&k_batch_begin<double>; }
 const void* batch_fold_f64() { return (const void*)&k_batch_fold<double>; }
 }  // namespace af
