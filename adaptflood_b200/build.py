@@ -44,7 +44,7 @@ UNITS = [
     ("af_xfer.cu", EXACT),
 ]
 HOST_UNITS = ["af_io.cpp", "af_arena.cpp", "af_output.cpp"]
-HEADERS = ["af_common.cuh", "af_pow.cuh", "af_pow_tables.h", "af_face64.cuh", "af_resident.cuh", "af_step.cuh", "af_simcore.cuh", "af_arena.h", "af_output.h",
+HEADERS = ["af_common.cuh", "af_pow.cuh", "af_pow_tables.h", "af_face64.cuh", "af_exchange.cuh", "af_resident.cuh", "af_stream.cuh", "af_step.cuh", "af_simcore.cuh", "af_arena.h", "af_output.h",
            "af_xfer.h"]
 
 

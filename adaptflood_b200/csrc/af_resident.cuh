@@ -8,16 +8,6 @@
 // per SM keeps a band of rows in shared memory and exchanges with the others
 // only its first and last rows' new H and Qx and its Hmax.
 //
-// Exchange.  Every 8 bytes that cross blocks carry 4 bytes of data and the
-// step's tag, so a reader polls the data itself and no fence, flag or atomic
-// stands between a step's last store and the next step's first use (an
-// 8-byte aligned access is not torn).  Buffers alternate between two copies:
-// a block writes step n+2's only after it has read every block's Hmax of
-// step n+1, which each sends after it has read step n's.  All blocks derive
-// the same dt, time and loop decisions from the same Hmax, so nothing else is
-// shared.  Every wait is bounded; a block that gives up flags the control
-// block and leaves, and so then do the others.
-//
 // Work.  A warp marches 32 columns down some rows, as the strip kernels do but
 // without halo lanes: the left neighbours come from shared memory, and the
 // faces on the strip's east side, for all its rows at once (a lane each),
@@ -26,9 +16,7 @@
 // so results are the same bit for bit.
 #pragma once
 
-#include <type_traits>
-
-#include "af_step.cuh"
+#include "af_exchange.cuh"
 
 namespace af {
 
@@ -36,13 +24,9 @@ struct ResidentParams {
   const int* row_off;       // special cells by row (CSR over rows, sorted by column)
   const SpecCell* row_spec;
   uint4* halo;              // [2][blocks][2][W][halo_words]
-  void* slot;               // [2][to][from] Hmax words, see post_max
-  double* part;             // [2][blocks][2] volume and area at mass-report steps
-  unsigned* tag;            // first unused tag
   int nr_max;               // rows of the tallest band
   int gy;                   // row groups a band is cut into (at most 32 rows each)
-  double t_stop;
-  long long max_steps;
+  LoopParams loop;
 };
 
 template <typename T>
@@ -68,36 +52,19 @@ __host__ __device__ inline size_t resident_smem(int nx, int nr, int gy) {
   return (W * (size_t)(7 * nr + 12) + 4) * sizeof(T) + 16 + nsx * (16 * (size_t)gy + 8 * (size_t)nr);
 }
 
-// Row groups of a band for `warps` warps: every group costs its rows and about
-// one and a half more (its first loads and the faces above and beside it).
-inline int resident_groups(int nx, int nr, int warps) {
+// Rows the busiest of a block's warps marches when a band of nr rows is cut
+// into g groups: every group costs about one and a half more than its rows (its
+// first loads and the faces above and beside it).
+inline double resident_cost(int nx, int nr, int warps, int g) {
   const int nsx = (nx + 31) / 32;
-  int best = 1;
-  double cost = 1e300;
-  for (int g = 1; g <= nr; g++) {
-    const int rows = (nr + g - 1) / g;
-    if (rows > 32) continue;
-    const double c = (double)((nsx * g + warps - 1) / warps) * (rows + 1.5);
-    if (c < cost) {
-      cost = c;
-      best = g;
-    }
-  }
+  return (double)((nsx * g + warps - 1) / warps) * ((nr + g - 1) / g + 1.5);
+}
+// The number of groups that costs least; a group has at most 32 rows.
+inline int resident_groups(int nx, int nr, int warps) {
+  int best = (nr + 31) / 32;
+  for (int g = best + 1; g <= nr; g++)
+    if (resident_cost(nx, nr, warps, g) < resident_cost(nx, nr, warps, best)) best = g;
   return best;
-}
-
-__device__ inline uint4 ld_relaxed(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p)
-               : "memory");
-  return v;
-}
-__device__ inline void st_relaxed(uint4* p, uint4 v) {
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y),
-               "r"(v.z), "r"(v.w)
-               : "memory");
 }
 
 __device__ inline void halo_put(uint4* at, float h, float q, unsigned tag) {
@@ -216,123 +183,6 @@ __device__ inline T add_source(T h, double v, double dx, double dA, double dt) {
   if (h < T(0)) h = T(0);
   return h;
 }
-// The segment k of the rain series that interp_series interpolates in at t
-// (times[k] <= t < times[k + 1], t inside the series), or -1.
-static __device__ __noinline__ int rain_segment(const StepParams& p, double t) {
-  const double* times = p.rain_times;
-  const int n = p.n_rain;
-  if (!p.rain_sorted || n < 2 || !(t > times[0] && t < times[n - 1])) return -1;
-  int lo = 0, hi = n - 1;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (times[mid] <= t) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// Largest of a warp's ordered 64-bit images (ord_encode).
-__device__ __forceinline__ unsigned long long warp_max_ord(unsigned long long v) {
-  const unsigned hi = (unsigned)(v >> 32);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)v : 0u);
-  return ((unsigned long long)mh << 32) | ml;
-}
-
-__device__ inline float cell_update(float h, float qw, float qe, float qn, float qs, bool rain,
-                                    const StepScal<float>& sc) {
-  // The operations of update_cells<float>, one cell in a pair.
-  const float2 a = __ffma2_rn(f2(qe, qs), f2(-1.0f, -1.0f), f2(qw, qn));
-  const float2 d = __fadd2_rn(f2(a.x, 0.0f), f2(a.y, 0.0f));
-  const float2 inc = __ffma2_rn(f2(sc.dt_dA, 0.0f), d, f2(rain ? sc.rain_depth : 0.0f, 0.0f));
-  return fmaxf(__fadd2_rn(f2(h, 0.0f), inc).x, 0.0f);
-}
-__device__ inline double cell_update(double h, double qw, double qe, double qn, double qs,
-                                     bool rain, const StepScal<double>& sc) {
-  return update_cell(h, qw, qe, qn, qs, rain, sc.rain_depth, sc.dtT, sc.dAT, sc.ph);
-}
-
-// Hmax of all blocks: each writes its own (the depth's ordered image with the
-// step's tag beside every 4 bytes) into every block's row and polls only its
-// own row, one warp per block.  Cycles per exchange of 148 blocks by itself:
-// 2900 with 8-byte words (FP32), 3700 with 16-byte words (FP64); all polling
-// one shared row 5800, two rounds in groups of 13 4100; an atomic maximum with
-// a counted arrival 3000, but 5000 in the loop, where its release also waits
-// for the halo stores.
-__device__ inline unsigned ord32(float x) {
-  const unsigned u = __float_as_uint(x);
-  return u & 0x80000000u ? ~u : u | 0x80000000u;
-}
-__device__ inline float ord32_value(unsigned u) {
-  return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
-}
-struct MaxF32 {
-  using Bits = unsigned;
-  using Word = uint2;
-  __device__ static Bits of(float m) { return ord32(m); }
-  __device__ static double value(Bits b) { return (double)ord32_value(b); }
-  __device__ static Bits warp(Bits b) { return __reduce_max_sync(0xffffffffu, b); }
-  __device__ static void put(Word* p, Bits b, unsigned tag) {
-    asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(b), "r"(tag)
-                 : "memory");
-  }
-  __device__ static bool get(const Word* p, Bits& b, unsigned tag) {
-    unsigned t;
-    asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(b), "=r"(t) : "l"(p)
-                 : "memory");
-    return t == tag;
-  }
-};
-struct MaxF64 {
-  using Bits = unsigned long long;
-  using Word = uint4;
-  __device__ static Bits of(double m) { return ord_encode(m); }
-  __device__ static double value(Bits b) { return ord_decode(b); }
-  __device__ static Bits warp(Bits b) { return warp_max_ord(b); }
-  __device__ static void put(Word* p, Bits b, unsigned tag) {
-    st_relaxed(p, make_uint4((unsigned)b, tag, (unsigned)(b >> 32), tag));
-  }
-  __device__ static bool get(const Word* p, Bits& b, unsigned tag) {
-    const uint4 x = ld_relaxed(p);
-    b = ((Bits)x.z << 32) | x.x;
-    return (x.y == tag) & (x.w == tag);
-  }
-};
-template <typename T>
-using MaxOf = typename std::conditional<sizeof(T) == 8, MaxF64, MaxF32>::type;
-
-template <typename M>
-__device__ __forceinline__ void post_max(void* slot, int nb, int buf, int b, unsigned tag,
-                                         typename M::Bits v) {
-  typename M::Word* const to = static_cast<typename M::Word*>(slot) + (size_t)buf * nb * nb + b;
-  for (int k = threadIdx.x & 31; k < nb; k += 32) M::put(to + (size_t)k * nb, v, tag);
-}
-// False when a wait ran out.
-template <typename M>
-__device__ __forceinline__ bool collect_max(void* slot, int nb, int buf, int b, unsigned tag,
-                                            typename M::Bits& v) {
-  constexpr int K = 5;  // loads in flight per lane: one round on up to 160 blocks
-  const typename M::Word* const row =
-      static_cast<const typename M::Word*>(slot) + ((size_t)buf * nb + b) * nb;
-  const int lane = threadIdx.x & 31;
-  typename M::Bits m = 0;
-  bool ok = true;
-  for (int k0 = lane; k0 - lane < nb; k0 += 32 * K) {
-    typename M::Bits x[K];
-    bool all = false;
-    for (int w = 0; w < (int)kRingWaitLimit && !all; w++) {
-      all = true;
-#pragma unroll
-      for (int u = 0; u < K; u++) all &= M::get(row + min(k0 + 32 * u, nb - 1), x[u], tag);
-    }
-    ok &= all;
-#pragma unroll
-    for (int u = 0; u < K; u++) m = x[u] > m ? x[u] : m;
-  }
-  v = M::warp(m);
-  return __all_sync(0xffffffffu, ok);
-}
-
 // A special cell's new depth: its sources, the update, its boundary depth.  `e`
 // is its entry; src (by source) and bc its band's values, or null.
 template <typename T>
@@ -346,29 +196,18 @@ static __device__ __noinline__ T special_cell(const StepParams& p, const StepSca
   return h;
 }
 
-// What warp 0 carries from step to step, in shared memory so that it takes no
-// registers of the march.
-struct Clock {
-  double t, dt_last, hmax, rate, next_mass;
-  double r_t0, r_t1, r_v0, r_v1;  // the rain series' segment of the last look-up
-  int status, mass_count;
-};
-
 template <typename T>
 __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
     k_resident(const __grid_constant__ StepParams p, const __grid_constant__ ResidentParams rp) {
   constexpr int NT = ResidentShape<T>::threads, NW = NT / 32;
   constexpr int HW = ResidentShape<T>::halo_words;
   extern __shared__ __align__(16) unsigned char s_mem[];
-  __shared__ StepScal<T> s_sc;
-  using M = MaxOf<T>;
-  __shared__ typename M::Bits s_max[NW];
-  __shared__ double s_v[NW], s_a[NW];
-  __shared__ int s_done, s_fail, s_nseg;
+  static_assert(NW == kLoopWarps, "one warp, one hand-in");
+  __shared__ LoopShared<T> S;
+  __shared__ int s_nseg;
   __shared__ double s_src[kBandSources];  // the band's sources' values at the step's time
   __shared__ T s_bc[kBandSpecials];       // and its special cells' boundary depths
   __shared__ SpecCell s_spec[kBandSpecials];
-  __shared__ Clock s_clock;
   SimCtl* ctl = p.ctl;
   int lane;  // read once: not recomputed from the thread index in the loop
   asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
@@ -392,25 +231,14 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
       s_mem + ((((size_t)W * (7 * rp.nr_max + 12) + 4) * sizeof(T) + 15) & ~(size_t)15));
   uint2* const at32 = reinterpret_cast<uint2*>(segs + nsx * rp.gy);  // {mask, first entry}
 
-  // ---- the loop's start: time, Hmax and limits, the same in every block
+  // ---- the loop's start, the same in every block
   const double t_start = ctl->t;
   const int par0 = ctl->parity;
-  const unsigned tag0 = *rp.tag;
+  const unsigned tag0 = *rp.loop.tag;
   long long n = 0;  // steps of this launch
-  const bool go = ctl->status == 0 && t_start < rp.t_stop && rp.max_steps > 0;
+  const bool go = ctl->status == 0 && t_start < rp.loop.t_stop && rp.loop.max_steps > 0;
   if (tid == 0) {
-    Clock& k = s_clock;
-    k.t = t_start;
-    k.dt_last = ctl->dt_last;
-    k.hmax = ctl->hmax;
-    k.rate = ctl->rain_rate;
-    k.next_mass = ctl->next_mass;
-    k.r_t0 = k.r_v0 = k.r_v1 = 0.0;
-    k.r_t1 = -1.0;
-    k.status = ctl->status;
-    k.mass_count = ctl->mass_count;
-    fill_scalars(p, k.t, step_dt(p, k.hmax), k.rate, k.next_mass, par0, s_sc);
-    s_fail = 0;
+    start_clock(p, S);
     // The band's marches: strip, first and last row.
     int q = 0;
     for (int gi = 0; gi < rp.gy; gi++) {
@@ -484,7 +312,7 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
   while (go) {
     const unsigned tag = tag0 + (unsigned)n;
     const int buf = (int)(n & 1);
-    const StepScal<T>& sc = s_sc;  // rewritten by the last warp once nobody needs it
+    const StepScal<T>& sc = S.sc;  // rewritten by warp 0 once nobody needs it
     const T* const H = H0 + buf * nH;
     T* const Hn = H0 + (buf ^ 1) * nH;
     const T* const X = X0 + buf * nH;
@@ -592,122 +420,10 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
         qn = qs;
       }
     }
-    const typename M::Bits mo = M::warp(M::of(m));
-    if (mass) {
-      v = warp_sum(v);
-      a = warp_sum(a);
-    }
-    if (lane == 0) {
-      s_max[warp] = mo;
-      s_v[warp] = v;
-      s_a[warp] = a;
-    }
+    hand_in(S, warp, m, v, a, mass);
     __syncthreads();
     if (warp == 0) {
-      // ---- Hmax of all blocks, then the next step's time, dt and constants
-      const typename M::Bits bm = M::warp(lane < NW ? s_max[lane] : 0);
-      if (mass) {
-        if (lane == 0) {
-          double sv = 0.0, sa = 0.0;
-          for (int w = 0; w < NW; w++) {
-            sv += s_v[w];
-            sa += s_a[w];
-          }
-          rp.part[(size_t)(buf * nb + b) * 2] = sv;
-          rp.part[(size_t)(buf * nb + b) * 2 + 1] = sa;
-          __threadfence();
-        }
-        __syncwarp();
-      }
-      post_max<M>(rp.slot, nb, buf, b, tag, bm);
-      // Time and rain rate while the others' Hmax is on its way.
-      Clock& ck = s_clock;
-      const double t = sc.t + sc.dt;
-      double rate = 0.0;
-      if (p.n_rain > 0) {
-        const double t0 = ck.r_t0, t1 = ck.r_t1;
-        if (t0 <= t && t < t1) {  // still in the segment: interp_series' own expression
-          const double v0 = ck.r_v0;
-          rate = v0 + (t - t0) / (t1 - t0) * (ck.r_v1 - v0);
-        } else {
-          const int k = rain_segment(p, t);
-          rate = interp_series(p.rain_times, p.rain_rates, p.n_rain, 0.0, t, p.rain_sorted != 0);
-          __syncwarp();
-          if (lane == 0) {
-            ck.r_t1 = -1.0;
-            if (k >= 0) {
-              ck.r_t0 = p.rain_times[k];
-              ck.r_t1 = p.rain_times[k + 1];
-              ck.r_v0 = p.rain_rates[k];
-              ck.r_v1 = p.rain_rates[k + 1];
-            }
-          }
-        }
-      }
-      typename M::Bits gm;
-      const bool ok = collect_max<M>(rp.slot, nb, buf, b, tag, gm);
-      const double gd = M::value(gm);
-      // The bookkeeping of fold_step, in every block alike.
-      const double hmax = gd > -(double)FLT_MAX ? gd : -DBL_MAX;
-      double next_mass = ck.next_mass;
-      int mass_count = ck.mass_count;
-      if (mass) {
-        if (b == 0 && mass_count < ctl->mass_cap) {
-          __threadfence();
-          const double* part = rp.part + (size_t)buf * nb * 2;
-          double s = 0.0, cs = 0.0, ar = 0.0;
-          for (int k = lane; k < nb; k += 32) {
-            kahan_add(s, cs, __ldcg(&part[2 * k]));
-            ar += __ldcg(&part[2 * k + 1]);
-          }
-          double S = 0.0, C = 0.0, A = 0.0;
-          for (int l = 0; l < 32; l++) {
-            kahan_add(S, C, __shfl_sync(0xffffffffu, s, l));
-            C += __shfl_sync(0xffffffffu, cs, l);
-            A += __shfl_sync(0xffffffffu, ar, l);
-          }
-          if (lane == 0) {
-            p.mass_series[3 * mass_count] = t;
-            p.mass_series[3 * mass_count + 1] = S + C;
-            p.mass_series[3 * mass_count + 2] = A;
-          }
-          mass_count++;
-        }
-        next_mass += p.mass_int;
-      }
-      const double dt_last = sc.dt;
-      const bool bad = !(dt_last > 0.0) || !(t < 1.0e300) || !(hmax == hmax);
-      const int status = !ok ? 2 : bad ? 1 : 0;
-      const bool done = status != 0 || !(t < rp.t_stop) || n + 1 >= rp.max_steps;
-      __syncwarp();
-      if (lane == 0) {
-        if (!done) {
-          // The fields of fill_scalars that change from step to step.
-          const double dt = step_dt(p, hmax);
-          s_sc.t = t;
-          s_sc.dt = dt;
-          s_sc.mass = p.mass_int > 0.0 && (t + dt >= next_mass);
-          s_sc.rain_on = rate > 0.0;
-          s_sc.rain_depth = T(rate * dt);
-          s_sc.dtT = T(dt);
-          s_sc.ph.gdt = T(p.g * dt);
-          if (sizeof(T) == 4) {
-            s_sc.dt_dA = T(dt / p.dA);
-            s_sc.ph.gdt_fn2 = T(p.g * dt * p.fpn * p.fpn * p.dxinv);
-          } else {
-            s_sc.ph.fast = face_range_ok(p.dx, p.fpn, p.depth_thresh, p.max_hflow, p.g * dt);
-          }
-        }
-        if (!ok) s_fail = 1;
-        s_done = done;
-        ck.t = t;
-        ck.dt_last = dt_last;
-        ck.hmax = hmax;
-        ck.rate = rate;
-        ck.next_mass = next_mass;
-        ck.status = status;
-        ck.mass_count = mass_count;
-      }
+      step_clock<T, false>(p, rp.loop, S, tag, n);
     } else {
       if (cached && ne > 0) {  // for the next step's time
         const double at = sc.t + sc.dt;
@@ -750,15 +466,15 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
           }
         }
       }
-      if (!ok) s_fail = 1;
+      if (!ok) S.fail = 1;
     }
     __syncthreads();
     n++;
-    if (s_fail) {
+    if (S.fail) {
       failed = true;
       break;
     }
-    if (s_done) break;
+    if (S.done) break;
   }
 
   // ---- the state back to its planes, and the control block
@@ -780,26 +496,7 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
       }
     }
   }
-  if (b == 0 && tid == 0) {
-    const long long limit = 0x3FFFFFFFFFFFFFFFLL;
-    ctl->t_stop = rp.t_stop;
-    ctl->step_stop = rp.max_steps > limit - ctl->step ? limit : ctl->step + rp.max_steps;
-    ctl->step += n;
-    ctl->done = 1;
-    ctl->arrive = 0u;
-    if (n > 0) {
-      const Clock& k = s_clock;
-      ctl->t = k.t;
-      ctl->hmax = k.hmax;
-      ctl->dt_last = k.dt_last;
-      ctl->rain_rate = k.rate;
-      ctl->next_mass = k.next_mass;
-      ctl->mass_count = k.mass_count;
-      ctl->parity = par;
-      if (k.status != 0) atomicMax(&ctl->status, k.status);
-      *rp.tag = tag0 + (unsigned)n + 16u;
-    }
-  }
+  if (b == 0 && tid == 0) stop_clock(p, rp.loop, S, par0, tag0, n);
 }
 
 }  // namespace af

@@ -18,6 +18,7 @@
 
 #include "af_output.h"
 #include "af_resident.cuh"
+#include "af_stream.cuh"
 #include "af_simcore.cuh"
 #include "af_xfer.h"
 
@@ -250,12 +251,14 @@ struct Sim {
   DevBuf bc_type, bc_value, bc_off, bc_times, bc_vals, bc_sorted;
   DevBuf rain_times, rain_rates, spec_off, spec;
   DevBuf ctl, partials, mass_series;
-  bool resident = false;  // small grid: the whole loop in one launch (af_resident.cuh)
-  DevBuf row_off, row_spec, halo, slot, rpart, rtag;
-  size_t halo_bytes = 0, slot_bytes = 0;
+  // The whole loop in one cooperative launch of `loop_blocks` blocks: the state
+  // on chip (resident) or in HBM (stream); neither: the step kernel in a graph.
+  bool resident = false, stream = false;
+  DevBuf row_off, row_spec, exch;  // exch: slots, partials, tag and, resident, halos
+  size_t exch_bytes = 0;
   ResidentParams rprm{};
-  unsigned rblocks = 0;
-  size_t rsmem = 0;
+  unsigned loop_blocks = 0;
+  size_t loop_smem = 0;
   SimCtl* pinned_ctl = nullptr;
   StepParams prm{};
   dim3 grid, block;
@@ -319,18 +322,23 @@ static int pick_shape(Sim& s) {
   // strips that still fit in as many waves, so every block gets the same
   // number of strips and each is as short as it can be (measured against
   // powers of two: 512^2 +21 %, 2048^2 +6 %, 4096^2 +5 %).  The FP64 step is
-  // bound by its arithmetic, so its strips (30 columns wide) are as tall as
-  // still leaves several waves of them: us per step at the chosen height and
-  // its neighbours, 512^2 R4 22.2 (R2 23.0, R6 21.8), 1024^2 R8 43.2 (R4 45.8,
-  // R12 45.0), 1501x1100 R8 60.0 (R4 66.0, R16 61.3), 2731x2747 R24 196 (R8
-  // 215, R32 198), 4096^2 R32 414 (R16 437, R48 422).
+  // bound by its arithmetic, so on grids of up to 2^24 cells the height is the
+  // one (4 to 32) that gives the busiest warp the fewest rows, each strip
+  // counted with 1.2 rows more for its first loads and faces; us per step at
+  // that height and at others: 700^2 R8 20.6 (R4 21.8, R16 26.5), 1501x1100 R24
+  // 47.4 (R8 50.5, R32 53.0), 2731x2747 R18 191 (R8 208, R16 195), 4096^2 R32
+  // 414 (R16 417).
   const long long cells = (long long)s.c.nx * s.c.ny;
   s.R = 32;
   if (s.prec == AF_PREC_F64) {
-    if (cells <= (1LL << 19)) s.R = 4;
-    else if (cells <= (1LL << 21)) s.R = 8;
-    else if (cells <= (1LL << 22)) s.R = 16;
-    else if (cells <= (1LL << 23)) s.R = 24;
+    double best = 1e300;
+    for (int R = 4; R <= 32 && cells <= (1LL << 24); R++) {
+      const double c = (double)((tiles_for(R) + slots - 1) / slots) * (R + 1.2);
+      if (c <= best) {
+        best = c;
+        s.R = R;
+      }
+    }
   } else if (cells < (1LL << 20)) {
     // Small FP32 grids: one-row strips, the shortest chain per warp even at
     // slightly over one wave (ms per step, one row against the two-wave rule:
@@ -360,31 +368,9 @@ static int pick_shape(Sim& s) {
   return AF_OK;
 }
 
-// Whether the grid's state fits on chip, and the resident loop's bands.  The
-// strip kernels' switches (and host-driven launches) keep the strip kernels;
-// AF_SIM_RESIDENT=0/1 forces the choice where the state fits.
-static bool pick_resident(Sim& s) {
-  const char* force = getenv("AF_SIM_RESIDENT");
-  if (force && force[0] == '0') return false;
-  const char* direct = getenv("AF_SIM_DIRECT_LAUNCH");
-  if (direct && direct[0] && direct[0] != '0') return false;
-  if (!force && (getenv("AF_SIM_VARIANT") || getenv("AF_SIM_ROWS") || getenv("AF_SIM_TMA")))
-    return false;
-  int dev = 0, sms = 0, coop = 0, smem = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-      !coop)
-    return false;
-  const bool f64 = s.prec == AF_PREC_F64;
-  const int nb = std::min(sms, s.c.ny);
-  const int nr = (s.c.ny + nb - 1) / nb;
-  const int threads = f64 ? ResidentShape<double>::threads : ResidentShape<float>::threads;
-  const int gy = resident_groups(s.c.nx, nr, threads / 32);
-  const size_t need =
-      f64 ? resident_smem<double>(s.c.nx, nr, gy) : resident_smem<float>(s.c.nx, nr, gy);
-  const void* fn = f64 ? resident_kernel_f64() : resident_kernel_f32();
+// A whole-loop launch of `fn` with `need` bytes of dynamic shared memory in
+// blocks of 16 warps, one per SM, can be made.
+static bool can_loop(const void* fn, size_t need, int smem) {
   cudaFuncAttributes a;
   if (cudaFuncGetAttributes(&a, fn) != cudaSuccess || need + a.sharedSizeBytes > (size_t)smem)
     return false;
@@ -394,14 +380,60 @@ static bool pick_resident(Sim& s) {
     return false;
   }
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, need) != cudaSuccess ||
-      per_sm < 1)
-    return false;
-  s.rblocks = (unsigned)nb;
-  s.rsmem = need;
-  s.rprm.nr_max = nr;
-  s.rprm.gy = gy;
-  return true;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * kLoopWarps, need) ==
+             cudaSuccess &&
+         per_sm >= 1;
+}
+
+// How the time loop runs (see Sim::resident).  AF_SIM_LOOP=resident, stream or
+// graph forces the choice (resident only where the state fits); host-driven
+// launches and a forced launch shape keep the step kernel.
+static void pick_loop(Sim& s) {
+  const char* force = getenv("AF_SIM_LOOP");
+  const char* direct = getenv("AF_SIM_DIRECT_LAUNCH");
+  if (direct && direct[0] && direct[0] != '0') return;
+  if (force ? force[0] == 'g' : getenv("AF_SIM_VARIANT") != nullptr) return;
+  int dev = 0, sms = 0, coop = 0, smem = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      !coop)
+    return;
+  const bool f64 = s.prec == AF_PREC_F64;
+  if (force ? force[0] == 'r' : !getenv("AF_SIM_ROWS") && !getenv("AF_SIM_TMA")) {
+    const int nb = std::min(sms, s.c.ny);
+    const int nr = (s.c.ny + nb - 1) / nb;
+    const int gy = resident_groups(s.c.nx, nr, kLoopWarps);
+    const size_t need =
+        f64 ? resident_smem<double>(s.c.nx, nr, gy) : resident_smem<float>(s.c.nx, nr, gy);
+    // Where both fit: the resident step grows with its busiest warp's rows
+    // (12 of 16 us on an FP64 grid 640 wide, whose 20 strips take 16 warps two
+    // rounds), the streamed one with the cells.  Estimated us per step, fitted
+    // to 128^2 ... 1023x769 FP32 and 128^2 ... 700^2 FP64; measured resident /
+    // streamed: FP32 317x203 4.2 / 7.4, 512^2 5.4 / 8.8, 1023x769 10.2 / 13.3,
+    // 2000x220 10.9 / 9.8; FP64 317x203 7.6 / 11.7, 512^2 13.3 / 13.9, 640x512
+    // 17.9 / 15.1.
+    const double rows = resident_cost(s.c.nx, nr, kLoopWarps, gy);
+    const double mcells = 1e-6 * s.c.nx * s.c.ny;
+    const bool faster = f64 ? 2.5 + 1.9 * rows < 11.0 + 14.0 * mcells
+                            : 2.4 + 0.6 * rows < 7.0 + 8.0 * mcells;
+    if ((faster || force) &&
+        can_loop(f64 ? resident_kernel_f64() : resident_kernel_f32(), need, smem)) {
+      s.resident = true;
+      s.loop_blocks = (unsigned)nb;
+      s.loop_smem = need;
+      s.rprm.nr_max = nr;
+      s.rprm.gy = gy;
+      return;
+    }
+  }
+  const size_t need = f64 ? stream_smem<double>() : stream_smem<float>();
+  if (can_loop(f64 ? stream_kernel_f64(s.tma) : stream_kernel_f32(s.tma), need, smem)) {
+    s.stream = true;
+    s.loop_blocks = (unsigned)sms;
+    s.loop_smem = need;
+  }
 }
 
 // The tensor map of the field planes (see encode_field_planes).
@@ -519,43 +551,51 @@ static int write_ctl(Sim& s) {
   return AF_OK;
 }
 
-// The exchange of the resident loop as new: nothing posted, no tag used.
-static int reset_resident(Sim& s) {
-  AF_CUDA(cudaMemsetAsync(s.halo.p, 0, s.halo_bytes, s.st));
-  AF_CUDA(cudaMemsetAsync(s.slot.p, 0, s.slot_bytes, s.st));
-  static const unsigned first = 1u;  // 0 is never a step's tag
-  AF_CUDA(cudaMemcpyAsync(s.rprm.tag, &first, sizeof first, cudaMemcpyHostToDevice, s.st));
+// The loop's exchange as new: nothing posted, no tag used (0 never is).
+static int reset_loop(Sim& s) {
+  AF_CUDA(cudaMemsetAsync(s.exch.p, 0, s.exch_bytes, s.st));
+  static const unsigned first = 1u;
+  AF_CUDA(cudaMemcpyAsync(s.rprm.loop.tag, &first, sizeof first, cudaMemcpyHostToDevice, s.st));
   return AF_OK;
 }
 
-// The resident loop's workspaces and its special cells by row.
-static int setup_resident(Sim& s, std::vector<SpecCell> spec) {
-  std::sort(spec.begin(), spec.end(), [](const SpecCell& a, const SpecCell& b) {
-    return a.row != b.row ? a.row < b.row : a.col < b.col;
-  });
-  std::vector<int> off((size_t)s.c.ny + 1, 0);
-  for (const SpecCell& e : spec) off[e.row + 1]++;
-  for (int j = 0; j < s.c.ny; j++) off[j + 1] += off[j];
-  AF_TRY(upload(s.row_off, off, s.st));
-  AF_TRY(upload(s.row_spec, spec, s.st));
+// The loop's workspaces and, resident, the special cells by row.
+static int setup_loop(Sim& s, std::vector<SpecCell> spec) {
+  ResidentParams& r = s.rprm;
+  const size_t nb = s.loop_blocks;
+  size_t at = 0;
+  auto put = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 255) / 256 * 256;
+    return o;
+  };
   const size_t hw = s.prec == AF_PREC_F64 ? ResidentShape<double>::halo_words
                                           : ResidentShape<float>::halo_words;
-  s.halo_bytes = (size_t)4 * s.rblocks * (s.c.nx + 1) * hw * sizeof(uint4);
-  AF_TRY(alloc_field(s.halo, s.halo_bytes, 1));
-  s.slot_bytes = (size_t)2 * s.rblocks * s.rblocks * sizeof(uint4);
-  AF_TRY(alloc_field(s.slot, s.slot_bytes, 1));
-  AF_TRY(alloc_field(s.rtag, 1, sizeof(unsigned)));
-  AF_TRY(alloc_field(s.rpart, (size_t)4 * s.rblocks, 8));
-  ResidentParams& r = s.rprm;
-  r.row_off = (const int*)s.row_off.p;
-  r.row_spec = (const SpecCell*)s.row_spec.p;
-  r.halo = (uint4*)s.halo.p;
-  r.part = (double*)s.rpart.p;
-  r.slot = s.slot.p;
-  r.tag = (unsigned*)s.rtag.p;
-  AF_TRY(reset_resident(s));
-  // Pageable sources: wait until the copies have left host memory.
-  AF_CUDA(cudaStreamSynchronize(s.st));
+  const size_t slot = put(2 * nb * nb * sizeof(uint4)), part = put(4 * nb * sizeof(double)),
+               tag = put(sizeof(unsigned)),
+               halo = put(s.resident ? 4 * nb * (s.c.nx + 1) * hw * sizeof(uint4) : 0);
+  s.exch_bytes = at;
+  AF_TRY(alloc_field(s.exch, at, 1));
+  char* const base = (char*)s.exch.p;
+  r.loop.slot = base + slot;
+  r.loop.part = (double*)(base + part);
+  r.loop.tag = (unsigned*)(base + tag);
+  r.halo = (uint4*)(base + halo);
+  AF_TRY(reset_loop(s));
+  if (s.resident) {
+    std::sort(spec.begin(), spec.end(), [](const SpecCell& a, const SpecCell& b) {
+      return a.row != b.row ? a.row < b.row : a.col < b.col;
+    });
+    std::vector<int> off((size_t)s.c.ny + 1, 0);
+    for (const SpecCell& e : spec) off[e.row + 1]++;
+    for (int j = 0; j < s.c.ny; j++) off[j + 1] += off[j];
+    AF_TRY(upload(s.row_off, off, s.st));
+    AF_TRY(upload(s.row_spec, spec, s.st));
+    r.row_off = (const int*)s.row_off.p;
+    r.row_spec = (const SpecCell*)s.row_spec.p;
+    // Pageable sources: wait until the copies have left host memory.
+    AF_CUDA(cudaStreamSynchronize(s.st));
+  }
   return AF_OK;
 }
 
@@ -815,8 +855,8 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   p.partials = static_cast<double*>(s->partials.p);
   p.mass_series = static_cast<double*>(s->mass_series.p);
   p.use_cond = 0;
-  s->resident = pick_resident(*s);
-  if (s->resident) AF_TRY(setup_resident(*s, std::move(tb.spec)));
+  pick_loop(*s);
+  if (s->resident || s->stream) AF_TRY(setup_loop(*s, std::move(tb.spec)));
   else AF_TRY(build_graph(*s));
   AF_CUDA(cudaStreamSynchronize(s->st));
   *out = s.release();
@@ -826,15 +866,16 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
 static int launch(Sim& s, double t_stop, long long max_steps) {
   AF_CUDA(cudaSetDevice(s.device));
   SimCtl* ctl = static_cast<SimCtl*>(s.ctl.p);
-  if (s.resident) {
+  if (s.resident || s.stream) {
     const bool f64 = s.prec == AF_PREC_F64;
-    s.rprm.t_stop = t_stop;
-    s.rprm.max_steps = max_steps;
-    void* args[] = {&s.prm, &s.rprm};
-    AF_CUDA(cudaLaunchCooperativeKernel(
-        f64 ? resident_kernel_f64() : resident_kernel_f32(), dim3(s.rblocks),
-        dim3(f64 ? ResidentShape<double>::threads : ResidentShape<float>::threads), args, s.rsmem,
-        s.st));
+    s.rprm.loop.t_stop = t_stop;
+    s.rprm.loop.max_steps = max_steps;
+    void* rargs[] = {&s.prm, &s.rprm};
+    void* sargs[] = {&s.prm, &s.rprm.loop, &s.fields};
+    const void* fn = s.resident ? (f64 ? resident_kernel_f64() : resident_kernel_f32())
+                                : (f64 ? stream_kernel_f64(s.tma) : stream_kernel_f32(s.tma));
+    AF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(s.loop_blocks), dim3(32 * kLoopWarps),
+                                        s.resident ? rargs : sargs, s.loop_smem, s.st));
     return AF_OK;
   }
   if (s.use_cond) {
@@ -1398,7 +1439,7 @@ static int restore(Sim& s, const char* path) {
   ctl.status = 0;
   *s.pinned_ctl = ctl;
   // A loop that gave up may have left its exchange half done.
-  if (s.resident) AF_TRY(reset_resident(s));
+  if (s.resident || s.stream) AF_TRY(reset_loop(s));
   return write_ctl(s);
 }
 

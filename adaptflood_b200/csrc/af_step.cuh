@@ -1844,6 +1844,8 @@ const void* step_kernel_f64(int variant, bool tma = true);
 const void* step_kernel_f32(int variant, bool tma = true);
 const void* resident_kernel_f64();  // the resident loop (af_resident.cuh)
 const void* resident_kernel_f32();
+const void* stream_kernel_f64(bool tma);  // the loop in one launch (af_stream.cuh)
+const void* stream_kernel_f32(bool tma);
 const void* batch_kernel_f64(int variant);
 const void* batch_kernel_f32(int variant);
 // Begin and fold kernels of the batch loop (one block of kFoldThreads),

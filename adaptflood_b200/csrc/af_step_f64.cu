@@ -1,6 +1,7 @@
 // af_step_f64.cu -- FP64 instantiation of the fused step.  Compiled with
 // -fmad=false so each expression rounds as the reference's C++ does.
 #include "af_resident.cuh"
+#include "af_stream.cuh"
 
 namespace af {
 // Indices follow kStepVariant in af_step.cuh.
@@ -30,6 +31,9 @@ const void* batch_kernel_f64(int variant) {
     case 4: return (const void*)&k_batch_step<double, 2, 8>;
     default: return (const void*)&k_batch_step<double, 1, 16>;
   }
+}
+const void* stream_kernel_f64(bool tma) {
+  return tma ? (const void*)&k_stream<double, true> : (const void*)&k_stream<double, false>;
 }
 const void* resident_kernel_f64() { return (const void*)&k_resident<double>; }
 const void* batch_begin_f64() { return (const void*)&k_batch_begin<double>; }
