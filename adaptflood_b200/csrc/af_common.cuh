@@ -94,7 +94,9 @@ __host__ __device__ inline double interp_series(const double* times, const doubl
 struct Scratch {
   void* dev = nullptr;
   size_t bytes = 0;
-  void* pinned = nullptr;  // 4 KB of pinned host memory for small readbacks
+  void* pinned = nullptr;  // 4 KB of mapped pinned host memory for small results ...
+  void* mapped = nullptr;  // ... and its device address
+  void* step = nullptr;    // the device words of af_floodplain_q (StepOut)
 };
 int scratch_get(size_t bytes, Scratch** out);  // current device; caller holds scratch_lock()
 std::mutex& scratch_lock();

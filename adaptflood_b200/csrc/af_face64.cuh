@@ -72,7 +72,7 @@ __device__ __forceinline__ double sqrt_near(double x, bool& bad) {
 // Whether face_fast may be used for a step's constants: with the flow depth
 // between depth_thresh and max_hflow these keep every intermediate of the
 // face law inside the ranges above.
-__device__ __forceinline__ bool face_range_ok(double dx, double fn, double depth_thresh,
+__host__ __device__ __forceinline__ bool face_range_ok(double dx, double fn, double depth_thresh,
                                               double max_hflow, double gdt) {
   const double lo = 9.313225746154785e-10, hi = 1073741824.0;  // 2^-30, 2^30
   return dx >= lo && dx <= hi && depth_thresh >= lo && max_hflow <= hi && (fn == 0.0 || fn >= lo) &&
@@ -80,14 +80,15 @@ __device__ __forceinline__ bool face_range_ok(double dx, double fn, double depth
 }
 
 // The discharge through one wet face (src/kernels.cpp:60-84 with theta = 1;
-// the same operations in the same order), x = |Qvect|^2.  `bad` is set when an operand is
+// the same operations in the same order): x = |Qvect|^2, base = the old
+// discharge's part of the numerator.  `bad` is set when an operand is
 // out of range and the value must come from the library forms instead.  Ranges: dh is
 // 0 or a multiple of 2^-260 here (depths and beds that make a face wet above
 // 2^-30 are), so only its upper bound is tested; below x = 2^-500 the
 // friction term is under 2^-60 and the denominator is 1 whatever sqrt(x) is,
 // so x is raised to 2^-500 (its high word; the low word may stay).  A dry
 // face's value means nothing, nor does its `bad`.
-__device__ __forceinline__ double face_fast(double dh, double hflow, double x, double q0,
+__device__ __forceinline__ double face_fast(double dh, double hflow, double x, double base,
                                             double dx, double rh, double rl, double gdt, double fn,
                                             bool& bad) {
   bad = false;
@@ -95,7 +96,7 @@ __device__ __forceinline__ double face_fast(double dh, double hflow, double x, d
   const int xh = __double2hiint(x);
   const double xs = __hiloint2double(max(xh, (1023 - 500) << 20), __double2loint(x));
   const double gh = gdt * hflow;
-  const double num = (q0 + 0.0) - gh * Sf;
+  const double num = base - gh * Sf;
   const double den = 1.0 + div_near(gh * fn * fn * sqrt_near(xs, bad), pw::pow_depth(hflow), bad);
   const int top = max(__double2hiint(dh) & 0x7fffffff, xh);  // both below 2^100 (x >= 0 or NaN)
   const unsigned low = (unsigned)__double2hiint(num) << 1;    // num is 0 or at least 2^-900

@@ -1,5 +1,8 @@
 // af_plain.cu -- the drop-in layer: one CUDA kernel per function of the
 // reference's src/kernels.hpp, FP64, reference layout, synchronous calls.
+// A call is one wait: what a function decides on the device (dt) stays there
+// for the kernels after it, and results the host needs are stored to mapped
+// host memory by the kernel that has them.
 //
 // Compiled with -fmad=false: every expression below rounds exactly as the
 // reference's C++ does on the CPU.  The friction term's pow(hflow, 10/3)
@@ -13,7 +16,7 @@
 #include <vector>
 
 #include "af_common.cuh"
-#include "af_pow.cuh"
+#include "af_face64.cuh"
 
 namespace af {
 
@@ -46,7 +49,12 @@ int scratch_get(size_t bytes, Scratch** out) {
   AF_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return AF_EINVAL;
   Scratch& s = g_scratch.s[dev];
-  if (!s.pinned) AF_CUDA(cudaMallocHost(&s.pinned, 4096));
+  if (!s.pinned) {
+    void* h = nullptr;
+    AF_CUDA(cudaHostAlloc(&h, 4096, cudaHostAllocMapped));
+    s.pinned = h;
+    AF_CUDA(cudaHostGetDevicePointer(&s.mapped, s.pinned, 0));
+  }
   if (s.bytes < bytes) {
     if (s.dev) AF_CUDA(cudaFree(s.dev));
     s.dev = nullptr;
@@ -58,6 +66,16 @@ int scratch_get(size_t bytes, Scratch** out) {
       return AF_ENOMEM;
     }
     s.bytes = want;
+  }
+  if (!s.step) {  // the step's words, as the last block of k_hmax_dt leaves them
+    void* p = nullptr;
+    const unsigned long long fresh[4] = {ord_encode(-DBL_MAX), 0ull, 0ull, 0ull};
+    AF_CUDA(cudaMalloc(&p, sizeof fresh));
+    if (const cudaError_t e = cudaMemcpy(p, fresh, sizeof fresh, cudaMemcpyHostToDevice)) {
+      cudaFree(p);
+      return cuda_fail(e);
+    }
+    s.step = p;
   }
   *out = &s;
   return AF_OK;
@@ -72,28 +90,51 @@ __device__ inline double warp_max(double m) {
   return m;
 }
 
-// FindHmax of src/kernels.cpp:30-33: max H over cells with DEM != nodata.
-__global__ void k_hmax(const double* __restrict__ H, const double* __restrict__ DEM, long long n,
-                       double nodata, unsigned long long* __restrict__ acc) {
+// The time step of a floodplain_q call, worked out on the device.
+struct StepOut {
+  unsigned long long acc;  // Hmax so far (ordered image); reset by the last block
+  unsigned arrived;
+  double dt;
+};
+
+// FindHmax of src/kernels.cpp:30-33 (max H over cells with DEM != nodata) and
+// dt from it (:36-43): the last block to finish has both, leaves dt for the
+// face kernel and stores it to the host.  Reads are the cost (16 bytes a
+// cell); two cells per thread and trip keep enough of them in flight.
+__global__ void k_hmax_dt(const double* __restrict__ H, const double* __restrict__ DEM, long long n,
+                          double nodata, double thresh, double cfl, double dx, double g,
+                          double init_dt, StepOut* __restrict__ out, double* __restrict__ host_dt) {
   double m = -DBL_MAX;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    double h = H[i];
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (; i + stride < n; i += 2 * stride) {
+    const double h0 = H[i], h1 = H[i + stride], z0 = DEM[i], z1 = DEM[i + stride];
+    if (z0 != nodata && h0 > m) m = h0;
+    if (z1 != nodata && h1 > m) m = h1;
+  }
+  if (i < n) {
+    const double h = H[i];
     if (DEM[i] != nodata && h > m) m = h;
   }
   m = warp_max(m);
   __shared__ double sm[32];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) sm[w] = m;
   __syncthreads();
-  if (w == 0) {
-    m = lane < (int)(blockDim.x >> 5) ? sm[lane] : -DBL_MAX;
-    m = warp_max(m);
-    if (lane == 0) atomicMax(acc, ord_encode(m));
-  }
+  if (w != 0) return;
+  m = lane < (int)(blockDim.x >> 5) ? sm[lane] : -DBL_MAX;
+  m = warp_max(m);
+  if (lane != 0) return;
+  if (m > -DBL_MAX) atomicMax(&out->acc, ord_encode(m));
+  __threadfence();
+  if (atomicAdd(&out->arrived, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const double hmax = ord_decode(atomicExch(&out->acc, ord_encode(-DBL_MAX)));
+  out->arrived = 0u;
+  const double dt = hmax > thresh ? cfl * dx / sqrt(g * hmax) : init_dt;
+  out->dt = dt;
+  *host_dt = dt;
 }
-
-__global__ void k_set_u64(unsigned long long* p, unsigned long long v) { *p = v; }
 
 // ------------------------------------------------------------ face fluxes
 // getmax / getmin of src/types.hpp:14-15 (not fmax/fmin: NaN and signed-zero
@@ -101,12 +142,13 @@ __global__ void k_set_u64(unsigned long long* p, unsigned long long v) { *p = v;
 __device__ inline double gmax(double a, double b) { return (a > b) ? a : b; }
 __device__ inline double gmin(double a, double b) { return (a < b) ? a : b; }
 
-// Qx of src/kernels.cpp:46-93, one thread per interior x-face.
+// Qx of src/kernels.cpp:46-93, one thread per interior x-face (any theta).
 __global__ void k_qx(const double* __restrict__ H, const double* __restrict__ DEM,
                      double* __restrict__ Qx, const double* __restrict__ Qxold,
                      const double* __restrict__ Qyold, int xsz, int ysz, double dx, double FPn,
-                     double DepthThresh, double MaxHflow, double dt, double g, double theta,
-                     double nodata) {
+                     double DepthThresh, double MaxHflow, const StepOut* __restrict__ step,
+                     double g, double theta, double nodata) {
+  const double dt = step->dt;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= xsz - 1 || j >= ysz) return;
@@ -147,12 +189,13 @@ __global__ void k_qx(const double* __restrict__ H, const double* __restrict__ DE
   Qx[pq0] = Q;
 }
 
-// Qy of src/kernels.cpp:96-143, one thread per interior y-face.
+// Qy of src/kernels.cpp:96-143, one thread per interior y-face (any theta).
 __global__ void k_qy(const double* __restrict__ H, const double* __restrict__ DEM,
                      double* __restrict__ Qy, const double* __restrict__ Qxold,
                      const double* __restrict__ Qyold, int xsz, int ysz, double dx, double FPn,
-                     double DepthThresh, double MaxHflow, double dt, double g, double theta,
-                     double nodata) {
+                     double DepthThresh, double MaxHflow, const StepOut* __restrict__ step,
+                     double g, double theta, double nodata) {
+  const double dt = step->dt;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= xsz || j >= ysz - 1) return;
@@ -191,6 +234,74 @@ __global__ void k_qy(const double* __restrict__ H, const double* __restrict__ DE
     }
   }
   Qy[pq0] = Q;
+}
+
+// One face as the reference writes it (theta = 1), for operands outside
+// face_fast's range; `base` is its theta*q0 + 0.5*(1-theta)*(qup + qdown).
+__device__ __noinline__ double face_any(double dh, double hflow, double x, double base, double dx,
+                                        double gdt, double fn) {
+  const double Sf = -dh / dx;
+  const double numerator = base - (gdt * hflow * Sf);
+  const double denominator =
+      1.0 + gdt * hflow * fn * fn * fabs(sqrt(x)) / pw::pow_ref(hflow, 10.0 / 3.0);
+  return numerator / denominator * dx;
+}
+
+// Qx and Qy of src/kernels.cpp:46-143 for theta = 1 in one pass: a thread has
+// the face east of its cell and the one south of it, whose inputs overlap, and
+// their straight-line face laws (af_face64.cuh) overlap in the FP64 pipe, which
+// bounds the pass.  With theta = 1 the recomputation of :86-89 gives the same
+// discharge.  4.5 M wet cells, with the depth maximum: 180 us a call as two
+// kernels with library divisions and roots, 137 us so.
+__global__ void __launch_bounds__(256)
+    k_faces(const double* __restrict__ H, const double* __restrict__ DEM, double* __restrict__ Qx,
+            double* __restrict__ Qy, const double* __restrict__ Qxold,
+            const double* __restrict__ Qyold, int xsz, int ysz, double dx, double rh, double rl,
+            double fn, double thresh, double max_hflow, const StepOut* __restrict__ step, double g,
+            double nodata, bool in_range) {
+  const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int j = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (j >= ysz) return;  // whole warps
+  const double gdt = g * step->dt;
+  const bool fast = in_range && gdt >= 9.094947017729282e-13 && gdt <= 1.099511627776e12;  // 2^+-40
+  const int W = xsz + 1;
+  const bool ex = i < xsz - 1, ey = i < xsz && j < ysz - 1;
+  const int ic = min(i, xsz - 1), ie = min(i + 1, xsz - 1), js = min(j + 1, ysz - 1);
+  const double z = DEM[ic + j * xsz], h = H[ic + j * xsz];
+  const double zE = DEM[ie + j * xsz], hE = H[ie + j * xsz];
+  const double zS = DEM[ic + js * xsz], hS = H[ic + js * xsz];
+  const double y = z + h, yE = zE + hE, yS = zS + hS;
+  double fx = gmax(y, yE) - gmax(z, zE), fy = gmax(y, yS) - gmax(z, zS);
+  fx = gmin(gmax(fx, 0.0), max_hflow);
+  fy = gmin(gmax(fy, 0.0), max_hflow);
+  const bool v = z != nodata;
+  const bool wx = ex & v & (zE != nodata) & (fx > thresh);
+  const bool wy = ey & v & (zS != nodata) & (fy > thresh);
+  double qx = 0.0, qy = 0.0;
+  if (__any_sync(0xffffffffu, wx | wy)) {
+    // Old discharges: columns ic, ic + 1 of rows j, j + 1 (faces exist up to
+    // column xsz and row ysz), and the faces up- and downstream.
+    const int a = ic + j * W, b = a + W;
+    const double x0 = Qxold[a], x1 = Qxold[a + 1], x2 = Qxold[b], x3 = Qxold[b + 1];
+    const double v0 = Qyold[a], v1 = Qyold[a + 1], v2 = Qyold[b], v3 = Qyold[b + 1];
+    const double xd = (wx && ic < xsz - 2) ? Qxold[a + 2] : 0.0;
+    const double yd = (wy && j < ysz - 2) ? Qyold[b + W] : 0.0;
+    const double xu = ic > 0 ? x0 : 0.0, yu = j > 0 ? v0 : 0.0;
+    const double bx = x1 + 0.0 * (xu + xd), by = v2 + 0.0 * (yu + yd);
+    const double ax = (v0 + v1 + v2 + v3) / 4.0, ay = (x0 + x1 + x2 + x3) / 4.0;
+    const double sx = x1 * x1 + ax * ax, sy = v2 * v2 + ay * ay;
+    bool badx, bady;
+    const double rx = face_fast(y - yE, fx, sx, bx, dx, rh, rl, gdt, fn, badx);
+    const double ry = face_fast(y - yS, fy, sy, by, dx, rh, rl, gdt, fn, bady);
+    qx = wx ? rx : 0.0;
+    qy = wy ? ry : 0.0;
+    if (__any_sync(0xffffffffu, (badx & wx) | (bady & wy) | !fast)) {
+      if (wx) qx = face_any(y - yE, fx, sx, bx, dx, gdt, fn);
+      if (wy) qy = face_any(y - yS, fy, sy, by, dx, gdt, fn);
+    }
+  }
+  if (ex) Qx[(i + 1) + j * W] = qx;
+  if (ey) Qy[i + (j + 1) * W] = qy;
 }
 
 // BCs_GPU of src/kernels.cpp:149-256; blockIdx.y selects the side (W, E, N, S).
@@ -440,57 +551,113 @@ __global__ void k_sort_small(unsigned long long* __restrict__ keys, int n) {
   for (int k = threadIdx.x; k < n; k += blockDim.x) keys[k] = s[k];
 }
 
-// src/main.cpp:256-260 in file order per cell: one thread per distinct cell.
-__global__ void k_apply_sources(double* __restrict__ H, const unsigned long long* __restrict__ keys,
-                                const double* __restrict__ ps_flow, int n) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    unsigned long long key = keys[k];
-    if (key == ~0ULL) continue;
-    unsigned cell = (unsigned)(key >> 32);
-    if (k > 0 && (unsigned)(keys[k - 1] >> 32) == cell) continue;  // not the segment head
-    double h = H[cell];
-    for (int m = k; m < n && keys[m] != ~0ULL && (unsigned)(keys[m] >> 32) == cell; m++) {
-      h += ps_flow[(unsigned)(keys[m] & 0xffffffffu)];
-      if (h < 0.0) h = 0.0;
-    }
-    H[cell] = h;
+// The segment head k of the sorted keys applies its cell's entries:
+// src/main.cpp:256-260 in file order ...
+__device__ inline void apply_sources_at(double* H, const unsigned long long* keys,
+                                        const double* ps_flow, int n, int k) {
+  const unsigned long long key = keys[k];
+  if (key == ~0ULL) return;
+  const unsigned cell = (unsigned)(key >> 32);
+  if (k > 0 && (unsigned)(keys[k - 1] >> 32) == cell) return;  // not the segment head
+  double h = H[cell];
+  for (int m = k; m < n && keys[m] != ~0ULL && (unsigned)(keys[m] >> 32) == cell; m++) {
+    h += ps_flow[(unsigned)(keys[m] & 0xffffffffu)];
+    if (h < 0.0) h = 0.0;
   }
+  H[cell] = h;
+}
+// ... and src/kernels.cpp:261-274 with the last effective boundary winning.
+__device__ inline void apply_bcs_at(double* H, const unsigned long long* keys, const int* type,
+                                    const double* value, int n, int k) {
+  const unsigned long long key = keys[k];
+  if (key == ~0ULL) return;
+  const unsigned cell = (unsigned)(key >> 32);
+  if (k > 0 && (unsigned)(keys[k - 1] >> 32) == cell) return;
+  bool write = false;
+  double v = 0.0;
+  for (int m = k; m < n && keys[m] != ~0ULL && (unsigned)(keys[m] >> 32) == cell; m++) {
+    const unsigned b = (unsigned)(keys[m] & 0xffffffffu);
+    const int t = type[b];
+    if (t == 1) {
+      write = true;
+      v = 0.0;
+    } else if (t == 2 || t == 3) {
+      write = true;
+      v = value[b];
+    }
+  }
+  if (write) H[cell] = v;
 }
 
-// src/kernels.cpp:261-274 with the last effective boundary of a cell winning.
+__global__ void k_apply_sources(double* __restrict__ H, const unsigned long long* __restrict__ keys,
+                                const double* __restrict__ ps_flow, int n) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+    apply_sources_at(H, keys, ps_flow, n, k);
+}
 __global__ void k_apply_point_bcs(double* __restrict__ H, const unsigned long long* __restrict__ keys,
                                   const int* __restrict__ type, const double* __restrict__ value,
                                   int n) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    unsigned long long key = keys[k];
-    if (key == ~0ULL) continue;
-    unsigned cell = (unsigned)(key >> 32);
-    if (k > 0 && (unsigned)(keys[k - 1] >> 32) == cell) continue;
-    bool write = false;
-    double v = 0.0;
-    for (int m = k; m < n && keys[m] != ~0ULL && (unsigned)(keys[m] >> 32) == cell; m++) {
-      unsigned b = (unsigned)(keys[m] & 0xffffffffu);
-      int t = type[b];
-      if (t == 1) {
-        write = true;
-        v = 0.0;
-      } else if (t == 2 || t == 3) {
-        write = true;
-        v = value[b];
-      }
-    }
-    if (write) H[cell] = v;
-  }
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+    apply_bcs_at(H, keys, type, value, n, k);
 }
 
-// Sorts the point keys into scratch and returns the sorted array.
+// Point sources or depth BCs of up to kSmallSort entries by one block: keys,
+// their sort and the application in shared memory, the error flag straight to
+// the host.  (The keys, sort and apply kernels with a clear before and a copy
+// after them took 33 us a call, 19 us so.)
+template <bool kSources>
+__global__ void __launch_bounds__(1024)
+    k_points_small(double* __restrict__ H, const int* __restrict__ idx, int n, int ncells,
+                   const int* __restrict__ type, const double* __restrict__ value,
+                   int* __restrict__ host_err) {
+  __shared__ unsigned long long s[kSmallSort];
+  int m = 1;
+  while (m < n) m <<= 1;
+  bool off = false;
+  for (int k = threadIdx.x; k < m; k += blockDim.x) {
+    const int c = k < n ? idx[k] : -1;
+    const bool out = c < 0 || c >= ncells;
+    off |= out && k < n;
+    s[k] = out ? ~0ULL : ((unsigned long long)(unsigned)c << 32) | (unsigned)k;
+  }
+  const int any_off = __syncthreads_or(off);
+  for (int size = 2; size <= m; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int k = threadIdx.x; k < m; k += blockDim.x) {
+        const int p = k ^ stride;
+        if (p > k) {
+          const bool up = (k & size) == 0;
+          const unsigned long long a = s[k], b = s[p];
+          if ((a > b) == up) {
+            s[k] = b;
+            s[p] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    if constexpr (kSources) apply_sources_at(H, s, value, n, k);
+    else apply_bcs_at(H, s, type, value, n, k);
+  }
+  if (threadIdx.x == 0) *host_err = any_off;
+}
+
+// Threads of a k_points_small block.
+inline unsigned point_threads(int n) {
+  unsigned t = 32;
+  while (t < 1024 && t < (unsigned)n) t <<= 1;
+  return t;
+}
+
+// Sorts more than kSmallSort point keys into scratch and returns the sorted
+// array.
 int sort_point_keys(const int* idx, int n, int ncells, cudaStream_t st, Scratch** sc_out,
                     unsigned long long** sorted_out, int** err_out) {
   size_t cub_bytes = 0;
-  if (n > kSmallSort) {
-    cub::DeviceRadixSort::SortKeys(nullptr, cub_bytes, (unsigned long long*)nullptr,
-                                   (unsigned long long*)nullptr, n, 0, 64, st);
-  }
+  cub::DeviceRadixSort::SortKeys(nullptr, cub_bytes, (unsigned long long*)nullptr,
+                                 (unsigned long long*)nullptr, n, 0, 64, st);
   size_t keys_bytes = ((size_t)n * 8 + 255) & ~(size_t)255;
   size_t need = 256 + 2 * keys_bytes + cub_bytes;
   Scratch* sc = nullptr;
@@ -503,14 +670,8 @@ int sort_point_keys(const int* idx, int n, int ncells, cudaStream_t st, Scratch*
   AF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
   k_point_keys<<<grid_for(n, 256), 256, 0, st>>>(idx, n, ncells, k0, err);
   AF_CUDA(cudaGetLastError());
-  unsigned long long* sorted = k0;
-  if (n > kSmallSort) {
-    AF_CUDA(cub::DeviceRadixSort::SortKeys(tmp, cub_bytes, k0, k1, n, 0, 64, st));
-    sorted = k1;
-  } else if (n > 1) {
-    k_sort_small<<<1, 1024, 0, st>>>(k0, n);
-    AF_CUDA(cudaGetLastError());
-  }
+  AF_CUDA(cub::DeviceRadixSort::SortKeys(tmp, cub_bytes, k0, k1, n, 0, 64, st));
+  unsigned long long* sorted = k1;
   *sc_out = sc;
   *sorted_out = sorted;
   *err_out = err;
@@ -572,31 +733,35 @@ int af_floodplain_q(const double* H, const double* DEM, double* Qx, double* Qy,
   std::lock_guard<std::mutex> lk(scratch_lock());
   Scratch* sc = nullptr;
   AF_TRY(scratch_get(64, &sc));
-  unsigned long long* acc = (unsigned long long*)sc->dev;
-  double Hmax = -DBL_MAX;
-  if (n > 0) {
-    k_set_u64<<<1, 1, 0, st>>>(acc, ord_encode(-DBL_MAX));
-    k_hmax<<<grid_for(n, 256), 256, 0, st>>>(H, DEM, n, nodata, acc);
-    AF_CUDA(cudaGetLastError());
-    AF_CUDA(cudaMemcpyAsync(sc->pinned, acc, 8, cudaMemcpyDeviceToHost, st));
-    AF_CUDA(cudaStreamSynchronize(st));
-    Hmax = ord_decode(*(unsigned long long*)sc->pinned);
+  StepOut* const out = (StepOut*)sc->step;
+  if (n == 0) {  // no cell: Hmax is its identity (src/kernels.cpp:36-43)
+    *Tstep = -DBL_MAX > DepthThresh ? cfl * dx / sqrt(g * -DBL_MAX) : InitTstep;
+    return finish(st);
   }
-  double dt;  // src/kernels.cpp:36-43
-  if (Hmax > DepthThresh) dt = cfl * dx / sqrt(g * Hmax);
-  else dt = InitTstep;
-  *Tstep = dt;
-  if (xsz > 1 && ysz > 0) {
-    dim3 b(32, 8), gq((xsz - 1 + 31) / 32, (ysz + 7) / 8);
-    k_qx<<<gq, b, 0, st>>>(H, DEM, Qx, Qxold, Qyold, xsz, ysz, dx, FPn, DepthThresh, MaxHflow,
-                           dt, g, theta, nodata);
+  k_hmax_dt<<<grid_for(n, 512, 4), 256, 0, st>>>(H, DEM, n, nodata, DepthThresh, cfl, dx, g,
+                                                 InitTstep, out, (double*)sc->mapped);
+  if (theta == 1.0) {
+    const double dxinv = 1.0 / dx;
+    const bool in_range = face_range_ok(dx, FPn, DepthThresh, MaxHflow, 1.0);
+    const dim3 gq((xsz + 31) / 32, (ysz + 7) / 8);
+    k_faces<<<gq, 256, 0, st>>>(H, DEM, Qx, Qy, Qxold, Qyold, xsz, ysz, dx, dxinv,
+                                std::fma(-dx, dxinv, 1.0) / dx, FPn, DepthThresh, MaxHflow, out, g,
+                                nodata, in_range);
+  } else {
+    if (xsz > 1 && ysz > 0) {
+      dim3 b(32, 8), gq((xsz - 1 + 31) / 32, (ysz + 7) / 8);
+      k_qx<<<gq, b, 0, st>>>(H, DEM, Qx, Qxold, Qyold, xsz, ysz, dx, FPn, DepthThresh, MaxHflow,
+                             out, g, theta, nodata);
+    }
+    if (xsz > 0 && ysz > 1) {
+      dim3 b(32, 8), gq((xsz + 31) / 32, (ysz - 1 + 7) / 8);
+      k_qy<<<gq, b, 0, st>>>(H, DEM, Qy, Qxold, Qyold, xsz, ysz, dx, FPn, DepthThresh, MaxHflow,
+                             out, g, theta, nodata);
+    }
   }
-  if (xsz > 0 && ysz > 1) {
-    dim3 b(32, 8), gq((xsz + 31) / 32, (ysz - 1 + 7) / 8);
-    k_qy<<<gq, b, 0, st>>>(H, DEM, Qy, Qxold, Qyold, xsz, ysz, dx, FPn, DepthThresh, MaxHflow,
-                           dt, g, theta, nodata);
-  }
-  return finish(st);
+  AF_TRY(finish(st));
+  *Tstep = *(volatile double*)sc->pinned;
+  return AF_OK;
 }
 
 int af_bcs(double* Qx, double* Qy, const double* H, const double* DEM, int xsz, int ysz,
@@ -628,6 +793,13 @@ int af_apply_point_bcs(double* H, const int* bc_idx, const int* bc_type, const d
   cudaStream_t st = as_stream(stream);
   std::lock_guard<std::mutex> lk(scratch_lock());
   Scratch* sc;
+  if (num_bcs <= kSmallSort) {
+    AF_TRY(scratch_get(0, &sc));
+    k_points_small<false><<<1, point_threads(num_bcs), 0, st>>>(H, bc_idx, num_bcs, ncells, bc_type,
+                                                                bc_value, (int*)sc->mapped);
+    AF_TRY(finish(st));
+    return *(volatile int*)sc->pinned ? AF_ERANGE : AF_OK;
+  }
   unsigned long long* sorted;
   int* err;
   AF_TRY(sort_point_keys(bc_idx, num_bcs, ncells, st, &sc, &sorted, &err));
@@ -686,6 +858,13 @@ int af_add_point_sources(double* H, const int* ps_idx, const double* ps_flow, in
   cudaStream_t st = as_stream(stream);
   std::lock_guard<std::mutex> lk(scratch_lock());
   Scratch* sc;
+  if (num <= kSmallSort) {
+    AF_TRY(scratch_get(0, &sc));
+    k_points_small<true><<<1, point_threads(num), 0, st>>>(H, ps_idx, num, ncells, nullptr, ps_flow,
+                                                           (int*)sc->mapped);
+    AF_TRY(finish(st));
+    return *(volatile int*)sc->pinned ? AF_ERANGE : AF_OK;
+  }
   unsigned long long* sorted;
   int* err;
   AF_TRY(sort_point_keys(ps_idx, num, ncells, st, &sc, &sorted, &err));

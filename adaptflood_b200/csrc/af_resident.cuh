@@ -121,9 +121,9 @@ __device__ __forceinline__ void two_faces(const FaceIn<double>& a, const FaceIn<
   const double ma = (aa + ab + ac + ad) / 4.0, mb = (ba + bb + bc + bd) / 4.0;
   bool xa, xb;
   const double fa =
-      face_fast(ya0 - ya1, ha, a0 * a0 + ma * ma, a0, ph.dx, ph.rh, ph.rl, ph.gdt, ph.fn, xa);
+      face_fast(ya0 - ya1, ha, a0 * a0 + ma * ma, a0 + 0.0, ph.dx, ph.rh, ph.rl, ph.gdt, ph.fn, xa);
   const double fb =
-      face_fast(yb0 - yb1, hb, b0 * b0 + mb * mb, b0, ph.dx, ph.rh, ph.rl, ph.gdt, ph.fn, xb);
+      face_fast(yb0 - yb1, hb, b0 * b0 + mb * mb, b0 + 0.0, ph.dx, ph.rh, ph.rl, ph.gdt, ph.fn, xb);
   qa = wa ? fa : 0.0;
   qb = wb ? fb : 0.0;
   if (__any_sync(0xffffffffu, (xa & wa) | (xb & wb) | !ph.fast)) {

@@ -288,7 +288,7 @@ static __device__ __noinline__ double face_any64(double z0, double h0, double z1
   const double x = q0 * q0 + qy_avg * qy_avg;
   if (fast) {
     bool bad;
-    const double q = face_fast(dh, hflow, x, q0, dx, rh, rl, gdt, fn, bad);
+    const double q = face_fast(dh, hflow, x, q0 + 0.0, dx, rh, rl, gdt, fn, bad);
     if (!bad) return q;
   }
   const double Sf = -dh / dx;
@@ -1175,9 +1175,9 @@ __device__ __forceinline__ bool run_strip64(const StepParams& p, const StepScal<
     if (__any_sync(0xffffffffu, wet_w | wet_s | !ph.fast)) {
       const double aw = (qyL + qy + qyNL + qyN) / 4.0, as = (qx + qxR + qxN + qxNR) / 4.0;
       bool bw, bs;
-      const double fw = face_fast(yL - y, hw, qx * qx + aw * aw, qx, ph.dx, ph.rh, ph.rl, ph.gdt,
+      const double fw = face_fast(yL - y, hw, qx * qx + aw * aw, qx + 0.0, ph.dx, ph.rh, ph.rl, ph.gdt,
                                   ph.fn, bw);
-      const double fs = face_fast(y - yN, hs, qyN * qyN + as * as, qyN, ph.dx, ph.rh, ph.rl, ph.gdt,
+      const double fs = face_fast(y - yN, hs, qyN * qyN + as * as, qyN + 0.0, ph.dx, ph.rh, ph.rl, ph.gdt,
                                   ph.fn, bs);
       qw = wet_w ? fw : 0.0;
       qs = wet_s ? fs : 0.0;
