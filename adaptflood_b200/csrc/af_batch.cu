@@ -342,24 +342,12 @@ static int put_vec(Batch& b, char* base, size_t off, const std::vector<V>& v) {
 }
 
 // Caller FP64 rows -> a padded field in the arena (`dst` = the field's
-// allocation, front guard included), on the copy stream: FP64 in one 2-D copy,
-// FP32 through the staging buffer and a conversion kernel.
+// allocation, front guard included), on the copy stream through the batch's
+// staging buffer.
 template <typename T>
 static int put_padded(Batch& b, char* dst, const double* src, int rows, int width, int P) {
-  T* d = reinterpret_cast<T*>(dst) + kGuard;
-  if (sizeof(T) == 8) {
-    AF_CUDA(copy2d_h2d(d, (size_t)P * 8, src, (size_t)width * 8, (size_t)width * 8, rows, b.cst));
-  } else {
-    const int chunk = (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
-    for (int j = 0; j < rows; j += chunk) {
-      const int n = std::min(chunk, rows - j);
-      AF_CUDA(copy2d_h2d(b.stage, (size_t)width * 8, src + (size_t)j * width, (size_t)width * 8,
-                         (size_t)width * 8, n, b.cst));
-      k_pad_from_f64<<<grid_for((long long)n * width, 256, 8), 256, 0, b.cst>>>(
-          b.stage, n, width, reinterpret_cast<float*>(d) + (size_t)j * P, P);
-      AF_CUDA(cudaGetLastError());
-    }
-  }
+  AF_TRY(put_rows(reinterpret_cast<T*>(dst) + kGuard, P, src, rows, width, (size_t)width, b.stage,
+                  b.cst));
   AF_CUDA(cudaStreamSynchronize(b.cst));
   return AF_OK;
 }
@@ -662,23 +650,11 @@ static bool finished(const Batch& b, int slot) {
 }
 
 // A padded field (first element at src) -> caller FP64 rows at host pitch
-// hpitch, on the copy stream; FP32 is converted on the device first.
+// hpitch, on the copy stream through the batch's staging buffer.
 template <typename T>
 static int get_field(Batch& b, const char* src, int rows, int width, int P, double* dst,
                      size_t hpitch) {
-  if (sizeof(T) == 8) {
-    AF_CUDA(copy2d_d2h(dst, hpitch * 8, src, (size_t)P * 8, (size_t)width * 8, rows, b.cst));
-  } else {
-    const int chunk = (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
-    for (int j = 0; j < rows; j += chunk) {
-      const int n = std::min(chunk, rows - j);
-      k_dense_to_f64<<<grid_for((long long)n * width, 256, 8), 256, 0, b.cst>>>(
-          reinterpret_cast<const float*>(src) + (size_t)j * P, P, n, width, b.stage);
-      AF_CUDA(cudaGetLastError());
-      AF_CUDA(copy2d_d2h(dst + (size_t)j * hpitch, hpitch * 8, b.stage, (size_t)width * 8,
-                         (size_t)width * 8, n, b.cst));
-    }
-  }
+  AF_TRY(get_rows(reinterpret_cast<const T*>(src), P, dst, rows, width, hpitch, b.stage, b.cst));
   AF_CUDA(cudaStreamSynchronize(b.cst));
   return AF_OK;
 }

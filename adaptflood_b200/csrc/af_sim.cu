@@ -250,7 +250,8 @@ struct Sim {
   DevBuf src_type, src_value, src_off, src_times, src_vals, src_sorted;
   DevBuf bc_type, bc_value, bc_off, bc_times, bc_vals, bc_sorted;
   DevBuf rain_times, rain_rates, spec_off, spec;
-  DevBuf ctl, partials, mass_series;
+  DevBuf ctl, partials, mass_series, stage;
+  size_t stage_bytes = 0;
   // The whole loop in one cooperative launch of `loop_blocks` blocks: the state
   // on chip (resident) or in HBM (stream); neither: the step kernel in a graph.
   bool resident = false, stream = false;
@@ -452,55 +453,37 @@ static int alloc_field(DevBuf& b, size_t elems, int esize) {
   return AF_OK;
 }
 
-// Copies a host FP64 field with `rows` x `width` entries and host pitch
-// `hpitch` into the padded device field (converted to the sim precision).
 // Field transfers between the caller's FP64 host arrays (rows of `width`
-// values at host pitch `hpitch`) and a padded device field.  FP64 fields are
-// one 2-D copy.  FP32 fields go through a dense FP64 device staging buffer in
-// chunks of rows, converted by a kernel on the device, so the host does no
-// per-element work (and pinned host arrays move at full link bandwidth).
+// values at host pitch `hpitch`) and a padded device field, through the
+// simulation's staging buffer (made on first use, at most kStageBytes, or one
+// row, and kept).
+static int get_stage(Sim& s, int rows, int width) {
+  const size_t want = std::max((size_t)width * 8, std::min(kStageBytes, (size_t)rows * width * 8));
+  if (s.stage_bytes >= want) return AF_OK;
+  if (s.stage.p) AF_CUDA(cudaFree(s.stage.p));
+  s.stage.p = nullptr;
+  s.stage_bytes = 0;
+  AF_TRY(alloc_field(s.stage, want, 1));
+  s.stage_bytes = want;
+  return AF_OK;
+}
+
 static int put_field(Sim& s, DevBuf& b, const double* src, int rows, int width, size_t hpitch) {
-  char* dst = static_cast<char*>(b.p) + (size_t)kGuard * s.esize;
-  if (s.prec == AF_PREC_F64) {
-    AF_CUDA(copy2d_h2d(dst, (size_t)s.P * 8, src, hpitch * 8, (size_t)width * 8, rows, s.st));
-    AF_CUDA(cudaStreamSynchronize(s.st));
-    return AF_OK;
-  }
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
-  DevBuf stage;
-  AF_TRY(alloc_field(stage, (size_t)chunk * width, 8));
-  for (int j = 0; j < rows; j += chunk) {
-    const int n = std::min(chunk, rows - j);
-    AF_CUDA(copy2d_h2d(stage.p, (size_t)width * 8, src + (size_t)j * hpitch, hpitch * 8,
-                       (size_t)width * 8, n, s.st));
-    k_pad_from_f64<<<grid_for((long long)n * width, 256, 8), 256, 0, s.st>>>(
-        static_cast<const double*>(stage.p), n, width,
-        reinterpret_cast<float*>(dst) + (size_t)j * s.P, s.P);
-    AF_CUDA(cudaGetLastError());
-  }
+  AF_TRY(get_stage(s, rows, width));
+  double* const stage = static_cast<double*>(s.stage.p);
+  AF_TRY(s.prec == AF_PREC_F64
+             ? put_rows(s.buf<double>(b), s.P, src, rows, width, hpitch, stage, s.st)
+             : put_rows(s.buf<float>(b), s.P, src, rows, width, hpitch, stage, s.st));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }
 
 static int get_field(Sim& s, DevBuf& b, double* dst, int rows, int width, size_t hpitch) {
-  const char* src = static_cast<const char*>(b.p) + (size_t)kGuard * s.esize;
-  if (s.prec == AF_PREC_F64) {
-    AF_CUDA(copy2d_d2h(dst, hpitch * 8, src, (size_t)s.P * 8, (size_t)width * 8, rows, s.st));
-    AF_CUDA(cudaStreamSynchronize(s.st));
-    return AF_OK;
-  }
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
-  DevBuf stage;
-  AF_TRY(alloc_field(stage, (size_t)chunk * width, 8));
-  for (int j = 0; j < rows; j += chunk) {
-    const int n = std::min(chunk, rows - j);
-    k_dense_to_f64<<<grid_for((long long)n * width, 256, 8), 256, 0, s.st>>>(
-        reinterpret_cast<const float*>(src) + (size_t)j * s.P, s.P, n, width,
-        static_cast<double*>(stage.p));
-    AF_CUDA(cudaGetLastError());
-    AF_CUDA(copy2d_d2h(dst + (size_t)j * hpitch, hpitch * 8, stage.p, (size_t)width * 8,
-                       (size_t)width * 8, n, s.st));
-  }
+  AF_TRY(get_stage(s, rows, width));
+  double* const stage = static_cast<double*>(s.stage.p);
+  AF_TRY(s.prec == AF_PREC_F64
+             ? get_rows(s.buf<double>(b), s.P, dst, rows, width, hpitch, stage, s.st)
+             : get_rows(s.buf<float>(b), s.P, dst, rows, width, hpitch, stage, s.st));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }

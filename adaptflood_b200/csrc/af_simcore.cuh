@@ -14,10 +14,12 @@
 // Padding is zero and never read into an owned result.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "af_step.cuh"
+#include "af_xfer.h"
 
 namespace af {
 
@@ -179,21 +181,26 @@ __global__ void k_volume_int(const T* __restrict__ H, int nx, int ny, int P, dou
   }
 }
 
-// Dense FP64 rows <-> a padded FP32 field (pitch P), converted on the device:
-// transfers of FP32 state move the caller's FP64 values through a device
-// staging buffer in chunks, with no per-element host work.
+// Dense FP64 rows <-> a padded field (pitch P) in the state precision, on the
+// device: transfers move the caller's FP64 values through a dense device
+// staging buffer in chunks, with no per-element host work and no 2-D copies,
+// whose rows the copy engines move one by one (see copy_rows).
 constexpr size_t kStageBytes = 64u << 20;
+// FP64 rows at least this long go straight into the padded field.
+constexpr size_t kLongRow = 16384;
 
-static __global__ void k_pad_from_f64(const double* __restrict__ src, int rows, int width,
-                               float* __restrict__ dst, int P) {
+template <typename T>
+__global__ void k_pad_from_f64(const double* __restrict__ src, int rows, int width,
+                               T* __restrict__ dst, int P) {
   const long long n = (long long)rows * width;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
     const long long j = k / width, i = k - j * width;
-    dst[j * P + i] = (float)src[k];
+    dst[j * P + i] = (T)src[k];
   }
 }
-static __global__ void k_dense_to_f64(const float* __restrict__ src, int P, int rows, int width,
+template <typename T>
+__global__ void k_dense_to_f64(const T* __restrict__ src, int P, int rows, int width,
                                double* __restrict__ dst) {
   const long long n = (long long)rows * width;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
@@ -201,6 +208,47 @@ static __global__ void k_dense_to_f64(const float* __restrict__ src, int P, int 
     const long long j = k / width, i = k - j * width;
     dst[k] = (double)src[j * P + i];
   }
+}
+
+// Caller FP64 rows at host pitch `hpitch` -> a padded device field at `dst`, and
+// back, through `stage` (at least one row, kStageBytes or the field).
+template <typename T>
+int put_rows(T* dst, int P, const double* src, int rows, int width, size_t hpitch, double* stage,
+             cudaStream_t st) {
+  if (sizeof(T) == 8 && (size_t)width * 8 >= kLongRow) {
+    AF_CUDA(copy2d_h2d(dst, (size_t)P * 8, src, hpitch * 8, (size_t)width * 8, rows, st));
+    return AF_OK;
+  }
+  const int chunk =
+      (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
+  for (int j = 0; j < rows; j += chunk) {
+    const int n = std::min(chunk, rows - j);
+    AF_CUDA(copy2d_h2d(stage, (size_t)width * 8, src + (size_t)j * hpitch, hpitch * 8,
+                       (size_t)width * 8, n, st));
+    k_pad_from_f64<T><<<grid_for((long long)n * width, 256, 8), 256, 0, st>>>(
+        stage, n, width, dst + (size_t)j * P, P);
+    AF_CUDA(cudaGetLastError());
+  }
+  return AF_OK;
+}
+template <typename T>
+int get_rows(const T* src, int P, double* dst, int rows, int width, size_t hpitch, double* stage,
+             cudaStream_t st) {
+  if (sizeof(T) == 8 && (size_t)width * 8 >= kLongRow) {
+    AF_CUDA(copy2d_d2h(dst, hpitch * 8, src, (size_t)P * 8, (size_t)width * 8, rows, st));
+    return AF_OK;
+  }
+  const int chunk =
+      (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
+  for (int j = 0; j < rows; j += chunk) {
+    const int n = std::min(chunk, rows - j);
+    k_dense_to_f64<T><<<grid_for((long long)n * width, 256, 8), 256, 0, st>>>(
+        src + (size_t)j * P, P, n, width, stage);
+    AF_CUDA(cudaGetLastError());
+    AF_CUDA(copy2d_d2h(dst + (size_t)j * hpitch, hpitch * 8, stage, (size_t)width * 8,
+                       (size_t)width * 8, n, st));
+  }
+  return AF_OK;
 }
 
 }  // namespace af
