@@ -41,7 +41,12 @@ def _make(target: str, ref_dir: str = None) -> None:
 def reference_dir():
     """The reference checkout named by AF_REFERENCE_DIR, if it exists here."""
     d = os.environ.get("AF_REFERENCE_DIR")
-    return d if d and os.path.isdir(d) else None
+    return d if d and has_sources(d) else None
+
+
+def has_sources(d) -> bool:
+    """Whether `d` holds the reference's sources (a mount point may be empty)."""
+    return os.path.isfile(os.path.join(d, "src", "kernels.cpp"))
 
 
 def _stale(so: str, sources) -> bool:
@@ -56,7 +61,7 @@ def build(ref: bool = True, ref_dir: str = None) -> None:
     or AF_REFERENCE_DIR), the reference library and CLI."""
     _make("oracle")
     d = ref_dir or reference_dir()
-    if ref and d and os.path.isdir(d):
+    if ref and d and has_sources(d):
         _make("ref", d)
 
 
