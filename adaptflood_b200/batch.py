@@ -74,7 +74,8 @@ class Batch:
         _lib.check(self.lib.af_batch_set_rows(self.h, int(cls), int(rows)), "af_batch_set_rows")
 
     def set_balance(self, strips_per_warp: int) -> None:
-        """Load-adaptive strip height target (0 = off); see af_batch_set_balance."""
+        """Strips per warp to aim at instead of the estimated best strip height (0 = the
+        heights of the size classes as they are); see af_batch_set_balance."""
         _lib.check(self.lib.af_batch_set_balance(self.h, int(strips_per_warp)),
                    "af_batch_set_balance")
 

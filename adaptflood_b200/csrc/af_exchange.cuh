@@ -45,21 +45,6 @@ __device__ inline void st_relaxed(uint4* p, uint4 v) {
                : "memory");
 }
 
-// The segment k of the rain series that interp_series interpolates in at t
-// (times[k] <= t < times[k + 1], t inside the series), or -1.
-static __device__ __noinline__ int rain_segment(const StepParams& p, double t) {
-  const double* times = p.rain_times;
-  const int n = p.n_rain;
-  if (!p.rain_sorted || n < 2 || !(t > times[0] && t < times[n - 1])) return -1;
-  int lo = 0, hi = n - 1;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (times[mid] <= t) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
 // Largest of a warp's ordered 64-bit images (ord_encode).
 __device__ __forceinline__ unsigned long long warp_max_ord(unsigned long long v) {
   const unsigned hi = (unsigned)(v >> 32);
@@ -308,22 +293,7 @@ __device__ __forceinline__ void step_clock(const StepParams& p, const LoopParams
   __syncwarp();
   if (lane == 0) {
     if (!done) {
-      // The fields of fill_scalars that change from step to step.
-      const double dt = step_dt(p, hmax);
-      S.sc.t = t;
-      S.sc.dt = dt;
-      S.sc.parity ^= 1;
-      S.sc.mass = p.mass_int > 0.0 && (t + dt >= next_mass);
-      S.sc.rain_on = rate > 0.0;
-      S.sc.rain_depth = T(rate * dt);
-      S.sc.dtT = T(dt);
-      S.sc.ph.gdt = T(p.g * dt);
-      if (sizeof(T) == 4) {
-        S.sc.dt_dA = T(dt / p.dA);
-        S.sc.ph.gdt_fn2 = T(p.g * dt * p.fpn * p.fpn * p.dxinv);
-      } else {
-        S.sc.ph.fast = face_range_ok(p.dx, p.fpn, p.depth_thresh, p.max_hflow, p.g * dt);
-      }
+      fill_step(p, t, step_dt(p, hmax), rate, next_mass, sc.parity ^ 1, S.sc);
     }
     if (!ok) S.fail = 1;
     S.done = done;

@@ -364,14 +364,16 @@ int af_batch_query(af_batch* b);
 /* Waits for the launch; AF_ESTATE if the batch's state is invalid. */
 int af_batch_sync(af_batch* b);
 /* Steps until every member has finished or max_steps batch steps have run,
- * and waits.  With the load-adaptive strip height on, it launches once per
+ * and waits.  Unless strip heights are fixed (balance 0), it launches once per
  * scenario completion so the strips are re-cut for the members that remain. */
 int af_batch_run(af_batch* b, int64_t max_steps, int64_t* batch_steps);
-/* Load-adaptive strip height: before each launch, the strip height of every
- * active member is the tuned height of its size class, lowered (powers of
- * two, at least 2 rows) until the active members give each warp of the
- * persistent grid about strips_per_warp strips.  0 turns it off (default 4).
- * Results do not depend on it. */
+/* Strip heights.  By default every active member gets, before each launch, the
+ * height of the least estimated step time for the active members together,
+ * at most that of its size class where af_batch_set_rows has set one.  After
+ * this call with strips_per_warp > 0: the height of its size class, lowered
+ * (powers of two, at least 2 rows) until the active members give each warp of
+ * the persistent grid about strips_per_warp strips.  With 0: the height of its
+ * size class.  Results do not depend on it. */
 int af_batch_set_balance(af_batch* b, int strips_per_warp);
 
 /* Status of a slot as of the last sync.  *state: 0 running, 1 finished
