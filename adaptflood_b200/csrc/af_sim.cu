@@ -303,7 +303,7 @@ static int pick_shape(Sim& s) {
     if (k >= 0 && k < kStepVariants) s.variant = k;
   }
   s.WY = kStepVariant[s.variant].wy;
-  s.tma = tma_for(s.prec == AF_PREC_F64, (long long)s.c.nx * s.c.ny);
+  s.tma = tma_rows();
   const void* fn = step_fn(s);
   int per_sm = 0, dev = 0, sms = kSMs;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * s.WY, 0) != cudaSuccess ||
@@ -316,44 +316,42 @@ static int pick_shape(Sim& s) {
     const long long nsy = (s.c.ny + R - 1) / R;
     return (long long)s.nsx * ((nsy + s.WY - 1) / s.WY);
   };
-  // Rows per strip.  Large grids take 32 (measured best at 8192^2: taller
-  // strips lose DRAM locality between the warps running side by side, shorter
-  // ones pay their prologue row more often).  In FP32 a grid whose 32-row
-  // strips fill at most two waves of the resident blocks takes the shortest
-  // strips that still fit in as many waves, so every block gets the same
-  // number of strips and each is as short as it can be (measured against
-  // powers of two: 512^2 +21 %, 2048^2 +6 %, 4096^2 +5 %).  The FP64 step is
-  // bound by its arithmetic, so on grids of up to 2^24 cells the height is the
-  // one (4 to 32) that gives the busiest warp the fewest rows, each strip
-  // counted with 1.2 rows more for its first loads and faces; us per step at
-  // that height and at others: 700^2 R8 20.6 (R4 21.8, R16 26.5), 1501x1100 R24
-  // 47.4 (R8 50.5, R32 53.0), 2731x2747 R18 191 (R8 208, R16 195), 4096^2 R32
-  // 414 (R16 417).
+  // Rows per strip: the height that gives the busiest warp the fewest rows, each
+  // strip counted with 1.2 rows more for its first loads and faces, up to a
+  // limit.  us per step at that height and at others: FP32 1400^2 R8 16.4,
+  // 2500x1801 R17 30.6 (R8 30.3, R12 33.8, R32 39.9), 3072^2 R17 54 (R8 57, R32
+  // 72); FP64 700^2 R8 20.6 (R4 21.8, R16 26.5), 1501x1100 R24 47.4 (R8 50.5, R32
+  // 53.0), 2731x2747 R18 191 (R8 208, R16 195), 4096^2 R32 414 (R16 417).
+  // The FP32 limit is the L2's: strips side by side share the cache lines at
+  // their edges and strips one above the other a row, read from DRAM once only
+  // while what all warps work on at a time (their number x R rows x 120 columns x
+  // 28 bytes) stays in the 126 MB, with room for warps that are ahead: 5792^2 R10
+  // 168, R12 167, R14 175, R32 194; 8192^2 R6 338, R8 326, R10 328, R12 352,
+  // R32 388; 16384^2 R6 1380, R7 1370, R8 1380, R10 1460, R32 1630, mostly dry
+  // R6 1304, R7 1292, R8 1395, R32 1616.  Up to 2^23 cells taller strips cost
+  // nothing.
+  // FP64 is bound by its arithmetic (16384^2 R32 6259, R16 6457, R8 6928).
   const long long cells = (long long)s.c.nx * s.c.ny;
+  const bool f64 = s.prec == AF_PREC_F64;
   s.R = 32;
-  if (s.prec == AF_PREC_F64) {
+  if (!f64 && cells < (1LL << 20)) {
+    // Small FP32 grids: one-row strips, the shortest chain per warp even at
+    // slightly over one wave (ms per step in a graph of step kernels, one row
+    // against the shortest strips that fit in one wave: 512^2 0.0312 / 0.0369,
+    // 724^2 0.0372 / 0.0393; at 1024^2 and above the rule is as fast or faster).
+    s.R = 1;
+  } else if (!f64 || cells <= (1LL << 24)) {
+    const int lo = f64 ? 4 : 2;
+    const int hi = f64 || cells <= (1LL << 23) ? 32 : cells <= (1LL << 25) ? 16
+                   : cells <= (1LL << 27)      ? 8
+                                               : 7;
     double best = 1e300;
-    for (int R = 4; R <= 32 && cells <= (1LL << 24); R++) {
+    for (int R = lo; R <= hi; R++) {
       const double c = (double)((tiles_for(R) + slots - 1) / slots) * (R + 1.2);
       if (c <= best) {
         best = c;
         s.R = R;
       }
-    }
-  } else if (cells < (1LL << 20)) {
-    // Small FP32 grids: one-row strips, the shortest chain per warp even at
-    // slightly over one wave (ms per step, one row against the two-wave rule:
-    // 512^2 0.0312 / 0.0369, 724^2 0.0372 / 0.0393; at 1024^2 and above the
-    // rule is as fast or faster).
-    s.R = 1;
-  } else {
-    const long long waves = (tiles_for(32) + slots - 1) / slots;
-    if (waves <= 2) {
-      for (int R = 2; R < 32; R++)
-        if (tiles_for(R) <= waves * slots) {
-          s.R = R;
-          break;
-        }
     }
   }
   if (const char* r = getenv("AF_SIM_ROWS")) {  // strip height override (tuning sweeps)

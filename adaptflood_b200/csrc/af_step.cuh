@@ -686,8 +686,9 @@ struct LaneAcc {
 // per-column edge tests.  Returns false after a wait time-out, with the
 // copies in flight drained and the grid's status flagged.
 // kSplitND: FP32 grids without nodata cells take a copy of the row loop
-// without the nodata tests (the same results; the batch kernel uses it, the
-// single-grid kernel measured no faster with it).
+// without the nodata tests (the same results).  The batch kernel and the
+// streamed loop use it (us per step there: 1024^2 13.7 -> 13.1, 2500x1801 33.0
+// -> 30.6, 8192^2 351 -> 341); k_step measured no faster with it.
 // kTma: one tiled copy per row through `tmap` instead of four bulk copies.
 template <typename T, bool kSplitND = false, bool kTma = false>
 __device__ __forceinline__ bool run_strip(const StepParams& p, const StepScal<T>& sc, int sx,
@@ -1897,22 +1898,15 @@ __global__ void __launch_bounds__(32 * WY, MINB) k_batch_step(const BatchParams 
 }
 
 // Whether a single grid's step reads its rows with one tiled copy (TMA) per
-// row instead of four bulk copies: FP32 grids of at most kTmaMaxCellsF32
-// cells, FP64 grids of at most kTmaMaxCellsF64.  The tiled copies take fewer
-// instructions but read a few per cent more DRAM bytes, so they pay where the
-// step is bound by issue or latency and lose where it is bound by bandwidth.
-// Measured, ms per FP32 step with tiled against bulk copies: 3072^2 0.0835 /
-// 0.0868, 4096^2 0.1226 / 0.1273, 4608^2 0.1484 / 0.1507; 5120^2 0.1801 /
-// 0.1734, 5792^2 0.2262 / 0.2140, 8192^2 0.432 / 0.369.  FP64, wet grids:
-// 3-5 % faster at every size from 1024^2 to 16384^2 (8192^2 2.12 against
-// 2.21 ms), but 6 % slower on the mostly dry 16384^2 start of the ponds
-// configuration, where the FP64 step is bandwidth-bound too.
-// AF_SIM_TMA=0/1 forces the choice.
-constexpr long long kTmaMaxCellsF32 = 4700LL * 4700;
-constexpr long long kTmaMaxCellsF64 = 1LL << 26;
-inline bool tma_for(bool f64, long long cells) {
-  if (const char* v = getenv("AF_SIM_TMA")) return v[0] == '1';
-  return cells <= (f64 ? kTmaMaxCellsF64 : kTmaMaxCellsF32);
+// row instead of four bulk copies: fewer instructions, and at the strip heights
+// of pick_shape no more DRAM bytes.  us per step, tiled against bulk copies at the
+// best height of each: FP32 2500x1801 30.3 / 33.7, 4096^2 92 / 95, 5792^2 167 /
+// 179, 8192^2 326 / 330, 7000x11000 375 / 383, 16384^2 1370 / 1400, mostly dry
+// 1292 / 1426; FP64 8192^2 1587 / 1782, 16384^2 6259 / 6961, mostly dry 2977 /
+// 3742.  AF_SIM_TMA=0 takes bulk copies.
+inline bool tma_rows() {
+  const char* v = getenv("AF_SIM_TMA");
+  return !v || v[0] == '1';
 }
 
 // The tensor map of a grid's field planes: 8 planes (H0, DEM, Qx0, Qy0, H1,

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
         if constexpr (sizeof(T) == 8)
           ok = run_strip64<kTma>(p, sc, sx, sy, rings[warp], bar, pos, acc, &fields);
         else
-          ok = run_strip<T, false, kTma>(p, sc, sx, sy, rings[warp], bar, pos, acc, &fields);
+          ok = run_strip<T, true, kTma>(p, sc, sx, sy, rings[warp], bar, pos, acc, &fields);
       }
       if (!ok && lane == 0) S.fail = 1;
       hand_in(S, warp, acc.m_cell, acc.v, acc.a, sc.mass);
