@@ -42,7 +42,7 @@ namespace af {
 
 constexpr int kClasses = 32;  // size class = floor(log2(nx*ny))
 constexpr int kBatchMassCap = 1 << 16;
-constexpr int kAuto = -1;  // Batch::balance: strip heights by estimated time (auto_rows)
+constexpr int kAuto = -1;  // Batch::balance: strip heights by estimated time (retile)
 
 static int size_class(long long cells) {
   int c = 0;
@@ -50,7 +50,8 @@ static int size_class(long long cells) {
   return c;
 }
 
-// Default strip height per size class, used until a tuned table is set.
+// Strip height per size class until a tuned table is set, where the caller asks
+// for heights by size class (a balance of 0 or more; see retile).
 static int default_rows(int cls) {
   if (cls < 16) return 4;
   if (cls < 20) return 8;
@@ -350,7 +351,7 @@ static int put_vec(Batch& b, char* base, size_t off, const std::vector<V>& v) {
 template <typename T>
 static int put_padded(Batch& b, char* dst, const double* src, int rows, int width, int P) {
   AF_TRY(put_rows(reinterpret_cast<T*>(dst) + kGuard, P, src, rows, width, (size_t)width, b.stage,
-                  b.cst));
+                  kStageBytes, b.cst));
   AF_CUDA(cudaStreamSynchronize(b.cst));
   return AF_OK;
 }
@@ -693,7 +694,8 @@ static bool finished(const Batch& b, int slot) {
 template <typename T>
 static int get_field(Batch& b, const char* src, int rows, int width, int P, double* dst,
                      size_t hpitch) {
-  AF_TRY(get_rows(reinterpret_cast<const T*>(src), P, dst, rows, width, hpitch, b.stage, b.cst));
+  AF_TRY(get_rows(reinterpret_cast<const T*>(src), P, dst, rows, width, hpitch, b.stage,
+                  kStageBytes, b.cst));
   AF_CUDA(cudaStreamSynchronize(b.cst));
   return AF_OK;
 }

@@ -1,10 +1,12 @@
 // af_sim.cu -- the simulation layer: device-resident state, forcing tables,
-// special-cell lists, and the CUDA graph that runs the time loop of one grid.
+// special-cell lists, and the launch that runs the time loop of one grid.
 // The padded field layout is described in af_simcore.cuh.
 //
-// The time loop (src/main.cpp:227 `while (t < sim_time)`) is one graph
-// launch: a begin kernel sets the stop condition, then a conditional WHILE
-// node re-runs the step kernel until its last block clears the condition.
+// The time loop (src/main.cpp:227 `while (t < sim_time)`) is one launch: a
+// cooperative kernel that holds the state on chip (af_resident.cuh) or streams
+// it from HBM (af_stream.cuh); where neither can be launched, a graph, in which
+// a begin kernel sets the stop condition, then a conditional WHILE node re-runs
+// the step kernel until its last block clears the condition.
 #include <algorithm>
 #include <cerrno>
 #include <cmath>
@@ -453,35 +455,44 @@ static int alloc_field(DevBuf& b, size_t elems, int esize) {
 
 // Field transfers between the caller's FP64 host arrays (rows of `width`
 // values at host pitch `hpitch`) and a padded device field, through the
-// simulation's staging buffer (made on first use, at most kStageBytes, or one
-// row, and kept).
-static int get_stage(Sim& s, int rows, int width) {
-  const size_t want = std::max((size_t)width * 8, std::min(kStageBytes, (size_t)rows * width * 8));
-  if (s.stage_bytes >= want) return AF_OK;
-  if (s.stage.p) AF_CUDA(cudaFree(s.stage.p));
-  s.stage.p = nullptr;
-  s.stage_bytes = 0;
-  AF_TRY(alloc_field(s.stage, want, 1));
+// simulation's staging buffer (made on first use and kept: a field, at most
+// kStageBytes, less where the device has no more; none for long FP64 rows).
+static int get_stage(Sim& s) {
+  const bool f64 = s.prec == AF_PREC_F64;
+  if (s.stage.p || (f64 && (size_t)s.c.nx * 8 >= kLongRow)) return AF_OK;
+  size_t want = std::min(kStageBytes, (size_t)(s.c.ny + 1) * (s.c.nx + 1) * 8);
+  for (;; want /= 8) {
+    if (cudaMalloc(&s.stage.p, want) == cudaSuccess) break;
+    const cudaError_t e = cudaGetLastError();
+    s.stage.p = nullptr;
+    if (want < (64u << 10)) {
+      if (f64) return AF_OK;  // the direct copy
+      cuda_fail(e);
+      return AF_ENOMEM;
+    }
+  }
   s.stage_bytes = want;
   return AF_OK;
 }
 
 static int put_field(Sim& s, DevBuf& b, const double* src, int rows, int width, size_t hpitch) {
-  AF_TRY(get_stage(s, rows, width));
+  AF_TRY(get_stage(s));
   double* const stage = static_cast<double*>(s.stage.p);
+  const size_t cap = s.stage_bytes;
   AF_TRY(s.prec == AF_PREC_F64
-             ? put_rows(s.buf<double>(b), s.P, src, rows, width, hpitch, stage, s.st)
-             : put_rows(s.buf<float>(b), s.P, src, rows, width, hpitch, stage, s.st));
+             ? put_rows(s.buf<double>(b), s.P, src, rows, width, hpitch, stage, cap, s.st)
+             : put_rows(s.buf<float>(b), s.P, src, rows, width, hpitch, stage, cap, s.st));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }
 
 static int get_field(Sim& s, DevBuf& b, double* dst, int rows, int width, size_t hpitch) {
-  AF_TRY(get_stage(s, rows, width));
+  AF_TRY(get_stage(s));
   double* const stage = static_cast<double*>(s.stage.p);
+  const size_t cap = s.stage_bytes;
   AF_TRY(s.prec == AF_PREC_F64
-             ? get_rows(s.buf<double>(b), s.P, dst, rows, width, hpitch, stage, s.st)
-             : get_rows(s.buf<float>(b), s.P, dst, rows, width, hpitch, stage, s.st));
+             ? get_rows(s.buf<double>(b), s.P, dst, rows, width, hpitch, stage, cap, s.st)
+             : get_rows(s.buf<float>(b), s.P, dst, rows, width, hpitch, stage, cap, s.st));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }

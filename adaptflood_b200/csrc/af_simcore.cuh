@@ -211,42 +211,49 @@ __global__ void k_dense_to_f64(const T* __restrict__ src, int P, int rows, int w
 }
 
 // Caller FP64 rows at host pitch `hpitch` -> a padded device field at `dst`, and
-// back, through `stage` (at least one row, kStageBytes or the field).
+// back, through the `cap` bytes of `stage` (FP64: null takes the direct copy).
+// A row longer than that goes in parts.
 template <typename T>
 int put_rows(T* dst, int P, const double* src, int rows, int width, size_t hpitch, double* stage,
-             cudaStream_t st) {
-  if (sizeof(T) == 8 && (size_t)width * 8 >= kLongRow) {
+             size_t cap, cudaStream_t st) {
+  if (sizeof(T) == 8 && (!stage || (size_t)width * 8 >= kLongRow)) {
     AF_CUDA(copy2d_h2d(dst, (size_t)P * 8, src, hpitch * 8, (size_t)width * 8, rows, st));
     return AF_OK;
   }
-  const int chunk =
-      (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
-  for (int j = 0; j < rows; j += chunk) {
-    const int n = std::min(chunk, rows - j);
-    AF_CUDA(copy2d_h2d(stage, (size_t)width * 8, src + (size_t)j * hpitch, hpitch * 8,
-                       (size_t)width * 8, n, st));
-    k_pad_from_f64<T><<<grid_for((long long)n * width, 256, 8), 256, 0, st>>>(
-        stage, n, width, dst + (size_t)j * P, P);
-    AF_CUDA(cudaGetLastError());
+  const int part = (int)std::min<size_t>(width, cap / 8);
+  for (int i = 0; i < width; i += part) {
+    const int w = std::min(part, width - i);
+    const int chunk = (int)std::min<size_t>(rows, cap / (8 * (size_t)w));
+    for (int j = 0; j < rows; j += chunk) {
+      const int n = std::min(chunk, rows - j);
+      AF_CUDA(copy2d_h2d(stage, (size_t)w * 8, src + (size_t)j * hpitch + i, hpitch * 8,
+                         (size_t)w * 8, n, st));
+      k_pad_from_f64<T><<<grid_for((long long)n * w, 256, 8), 256, 0, st>>>(
+          stage, n, w, dst + (size_t)j * P + i, P);
+      AF_CUDA(cudaGetLastError());
+    }
   }
   return AF_OK;
 }
 template <typename T>
 int get_rows(const T* src, int P, double* dst, int rows, int width, size_t hpitch, double* stage,
-             cudaStream_t st) {
-  if (sizeof(T) == 8 && (size_t)width * 8 >= kLongRow) {
+             size_t cap, cudaStream_t st) {
+  if (sizeof(T) == 8 && (!stage || (size_t)width * 8 >= kLongRow)) {
     AF_CUDA(copy2d_d2h(dst, hpitch * 8, src, (size_t)P * 8, (size_t)width * 8, rows, st));
     return AF_OK;
   }
-  const int chunk =
-      (int)std::max<size_t>(1, std::min<size_t>(rows, kStageBytes / (8 * (size_t)width)));
-  for (int j = 0; j < rows; j += chunk) {
-    const int n = std::min(chunk, rows - j);
-    k_dense_to_f64<T><<<grid_for((long long)n * width, 256, 8), 256, 0, st>>>(
-        src + (size_t)j * P, P, n, width, stage);
-    AF_CUDA(cudaGetLastError());
-    AF_CUDA(copy2d_d2h(dst + (size_t)j * hpitch, hpitch * 8, stage, (size_t)width * 8,
-                       (size_t)width * 8, n, st));
+  const int part = (int)std::min<size_t>(width, cap / 8);
+  for (int i = 0; i < width; i += part) {
+    const int w = std::min(part, width - i);
+    const int chunk = (int)std::min<size_t>(rows, cap / (8 * (size_t)w));
+    for (int j = 0; j < rows; j += chunk) {
+      const int n = std::min(chunk, rows - j);
+      k_dense_to_f64<T><<<grid_for((long long)n * w, 256, 8), 256, 0, st>>>(
+          src + (size_t)j * P + i, P, n, w, stage);
+      AF_CUDA(cudaGetLastError());
+      AF_CUDA(copy2d_d2h(dst + (size_t)j * hpitch + i, hpitch * 8, stage, (size_t)w * 8,
+                         (size_t)w * 8, n, st));
+    }
   }
   return AF_OK;
 }

@@ -58,6 +58,16 @@ def test_round_trips_from_several_threads(cuda):
     assert not bad, bad
 
 
+def test_rows_longer_than_the_staging_buffer(cuda):
+    nx, ny = (64 << 20) // 8 + 1001, 2
+    h = np.random.default_rng(5).random((ny, nx)).astype(np.float32).astype(np.float64)
+    with Batch("f32", arena_bytes=2 << 30) as b:
+        k = b.add(sc.Case(nx, ny, 5.0, np.full((ny, nx), -50.0), h0=h, sim_time=0.0))
+        b.run()
+        np.testing.assert_array_equal(b.depth(k), h)
+    _round_trip(nx, ny, "f32", 5)
+
+
 def test_batch_members_round_trip(cuda):
     rng = np.random.default_rng(3)
     cases = []
