@@ -1,6 +1,6 @@
-// af_step.cuh -- the fused local-inertial time step (one kernel per step).
+// af_step.cuh -- the fused local-inertial time step (strips and kernels).
 //
-// One launch performs the whole body of the reference's time loop,
+// A step performs the whole body of the reference's time loop,
 // src/main.cpp:227-288: the CFL time step from the previous state's Hmax
 // (src/kernels.cpp:29-43), the interior face fluxes (:46-143), the edge faces
 // (:149-256), the point sources (src/main.cpp:245-262), rainfall
@@ -13,8 +13,7 @@
 // and R consecutive rows and marches down the rows.  Its 32 lanes each take N
 // consecutive cells (one double, or one 16-byte vector of 4 floats) of every
 // array; lanes 0 and 31 are halo lanes whose cells belong to the neighbouring
-// warps, so every x-neighbour a face needs is one warp shuffle away and the
-// warp never touches shared memory.  Each face flux is computed by the lane
+// warps, so every x-neighbour a face needs is one warp shuffle away.  Each face flux is computed by the lane
 // that owns the cell east (x-faces) or south (y-faces) of it, once per step,
 // except the face columns at strip edges and the face row above a strip,
 // which the neighbouring strip recomputes (identically) instead of waiting.
@@ -24,8 +23,11 @@
 // when a face is loaded, with the same rounding the reference's UpdateQs
 // uses, so no Qold arrays exist.
 //
+// The strips here run in three kernels: k_step below (one launch a step), the
+// streamed loop (af_stream.cuh: all steps in one launch) and k_batch_step.
+//
 // Control lives in device memory (SimCtl): time, Hmax, parity, step counters.
-// The last block to finish (one atomic counter, no waiting) folds Hmax,
+// In k_step the last block to finish (one atomic counter, no waiting) folds Hmax,
 // advances time, computes the next step's rain rate and decides whether the
 // loop continues (the condition of the enclosing CUDA-graph while node).
 #pragma once

@@ -15,8 +15,8 @@
  *    ends in Kokkos::fence().  The reference's functions return void and abort
  *    on error; these return AF_OK or a negative AF_E* code.
  *
- * 2. The simulation layer (af_sim_*): one fused, graph-launched kernel per
- *    time step with device-resident dt, time and hydrograph interpolation, in
+ * 2. The simulation layer (af_sim_*): the whole time loop in one launch of
+ *    fused steps with device-resident dt, time and hydrograph interpolation, in
  *    FP64 (results within 1e-9 m of the reference) or FP32 state with FP64
  *    time, interpolation and volume accumulation.
  *
