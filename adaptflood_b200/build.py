@@ -111,5 +111,16 @@ def build_wait_test(verbose: bool = False) -> str:
                  defines=("AF_RING_WAIT_LIMIT=0",))
 
 
+# A test build whose resident loop lets all warps but the block's first come
+# 20 us late past a step's barrier (the first has gone on to the next step by
+# then): what they read there must not be what the first rewrites.
+LATETEST_LIB = os.path.join(HERE, "libadaptflood_latetest.so")
+
+
+def build_late_test(verbose: bool = False) -> str:
+    return build(verbose=verbose, obj_dir=os.path.join(HERE, "_build_latetest"), lib=LATETEST_LIB,
+                 defines=("AF_LATE_NS=20000",))
+
+
 if __name__ == "__main__":
     print(build(verbose=False, ptxas_info="--ptxas" in sys.argv) or "up to date")

@@ -29,6 +29,14 @@ struct ResidentParams {
   LoopParams loop;
 };
 
+// Nanoseconds that the warps beside warp 0 are late past the march's barrier.  A
+// test build sets it, so that what they read there is read after warp 0 has
+// gone on to the next step.
+#ifndef AF_LATE_NS
+#define AF_LATE_NS 0
+#endif
+constexpr unsigned kLateNs = AF_LATE_NS;
+
 template <typename T>
 struct ResidentShape;
 template <>
@@ -312,7 +320,7 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
   while (go) {
     const unsigned tag = tag0 + (unsigned)n;
     const int buf = (int)(n & 1);
-    const StepScal<T>& sc = S.sc;  // rewritten by warp 0 once nobody needs it
+    const StepScal<T>& sc = S.sc;  // warp 0 rewrites it past the march's barrier
     const T* const H = H0 + buf * nH;
     T* const Hn = H0 + (buf ^ 1) * nH;
     const T* const X = X0 + buf * nH;
@@ -421,12 +429,14 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
       }
     }
     hand_in(S, warp, m, v, a, mass);
+    // The next step's time, read before the barrier: past it warp 0 rewrites sc.
+    const double at = sc.t + sc.dt;
     __syncthreads();
     if (warp == 0) {
       step_clock<T, false>(p, rp.loop, S, tag, n);
     } else {
-      if (cached && ne > 0) {  // for the next step's time
-        const double at = sc.t + sc.dt;
+      if constexpr (kLateNs > 0) __nanosleep(kLateNs);
+      if (cached && ne > 0) {
         for (int k = tid - 32; k < nsrc; k += NT - 32) s_src[k] = source_value(p, src0 + k, at);
         for (int e = tid - 32; e < ne; e += NT - 32)
           if (s_spec[e].bc >= 0) s_bc[e] = boundary_depth<T>(p, s_spec[e].bc, at);
