@@ -93,14 +93,16 @@ __device__ __forceinline__ double face_fast(double dh, double hflow, double x, d
                                             bool& bad) {
   bad = false;
   const double Sf = div_const(-dh, dx, rh, rl);
-  const int xh = __double2hiint(x) & 0x7fffffff;  // x >= 0 or a NaN of either sign
+  const int xh = __double2hiint(x);
   const double xs = __hiloint2double(max(xh, (1023 - 500) << 20), __double2loint(x));
   const double gh = gdt * hflow;
   const double num = base - gh * Sf;
   const double den = 1.0 + div_near(gh * fn * fn * sqrt_near(xs, bad), pw::pow_depth(hflow), bad);
-  const int top = max(__double2hiint(dh) & 0x7fffffff, xh);  // both below 2^100
+  // Both below 2^100.  x >= 0 or a NaN, which as an unsigned number is above
+  // with either sign.
+  const unsigned top = max((unsigned)__double2hiint(dh) & 0x7fffffffu, (unsigned)xh);
   const unsigned low = (unsigned)__double2hiint(num) << 1;    // num is 0 or at least 2^-900
-  bad = bad | (top >= (1023 + 100) << 20) | (low - 1u < ((unsigned)(1023 - 900) << 21) - 1u);
+  bad = bad | (top >= (1023u + 100u) << 20) | (low - 1u < ((unsigned)(1023 - 900) << 21) - 1u);
   return div_near(num, den, bad) * dx;
 }
 
