@@ -27,8 +27,12 @@ struct LoopParams {
   void* slot;     // [2][to][from] Hmax words, see post_max
   double* part;   // [2][blocks][2] volume and area at mass-report steps
   unsigned* tag;  // first unused tag
+  // The first launch of a call (more = 0) has the call's limits, those after it
+  // find them in the control block.  A launch ends after `slice` steps at most.
   double t_stop;
   long long max_steps;
+  int slice;
+  int more;
 };
 
 __device__ inline uint4 ld_relaxed(const uint4* p) {
@@ -151,6 +155,8 @@ __device__ __forceinline__ bool collect_max(void* slot, int nb, int buf, int b, 
 // registers of the step.
 struct Clock {
   double t, dt_last, hmax, rate, next_mass;
+  double t_stop;   // the call's
+  int most;        // steps of this launch
   double r_t0, r_t1, r_v0, r_v1;  // the rain series' segment of the last look-up
   int status, mass_count;
 };
@@ -163,14 +169,24 @@ struct LoopShared {
   typename MaxOf<T>::Bits max[kLoopWarps];
   double v[kLoopWarps], a[kLoopWarps];
   int done, fail;
+  int par0;       // the parity and first tag of this launch
+  unsigned tag0;
 };
 
+// Whether there is a step to take, the same in every block and thread.
+__device__ inline bool loop_goes(const SimCtl* ctl, const LoopParams& lp) {
+  return ctl->status == 0 && (lp.more ? !ctl->done : ctl->t < lp.t_stop && lp.max_steps > 0);
+}
+
 // The loop's start from the control block, the same in every block (one
-// thread); returns the time.
+// thread).
 template <typename T>
-__device__ inline void start_clock(const StepParams& p, LoopShared<T>& S) {
+__device__ inline void start_clock(const StepParams& p, const LoopParams& lp, LoopShared<T>& S) {
   const SimCtl* ctl = p.ctl;
   Clock& k = S.clock;
+  k.t_stop = lp.more ? ctl->t_stop : lp.t_stop;
+  const long long left = lp.more ? ctl->step_stop - ctl->step : lp.max_steps;
+  k.most = left < lp.slice ? (int)left : lp.slice;
   k.t = ctl->t;
   k.dt_last = ctl->dt_last;
   k.hmax = ctl->hmax;
@@ -181,8 +197,10 @@ __device__ inline void start_clock(const StepParams& p, LoopShared<T>& S) {
   k.status = ctl->status;
   k.mass_count = ctl->mass_count;
   fill_scalars(p, k.t, step_dt(p, k.hmax), k.rate, k.next_mass, ctl->parity, S.sc);
-  S.done = 0;
+  S.done = !loop_goes(ctl, lp);
   S.fail = 0;
+  S.par0 = ctl->parity;
+  S.tag0 = *lp.tag;
 }
 
 // One warp's share of the step: its largest valid depth (-FLT_MAX: none) and,
@@ -205,13 +223,14 @@ __device__ __forceinline__ void hand_in(LoopShared<T>& S, int warp, T m, double 
 // Warp 0 of every block, after the whole block's step n (tag `tag`): Hmax of
 // all blocks, then the next step's time, dt and constants.  kState: the state
 // went to global memory, so it must be there before the word that says so.
-template <typename T, bool kState>
+template <typename T, bool kState, typename N>
 __device__ __forceinline__ void step_clock(const StepParams& p, const LoopParams& lp,
-                                           LoopShared<T>& S, unsigned tag, long long n) {
+                                           LoopShared<T>& S, unsigned tag, N n) {
   using M = MaxOf<T>;
   constexpr int NW = kLoopWarps;
   const int lane = threadIdx.x & 31, nb = gridDim.x, b = blockIdx.x, buf = (int)(n & 1);
   const StepScal<T>& sc = S.sc;
+  Clock& ck = S.clock;
   const bool mass = sc.mass;
   const typename M::Bits bm = M::warp(lane < NW ? S.max[lane] : 0);
   if (mass) {
@@ -227,11 +246,24 @@ __device__ __forceinline__ void step_clock(const StepParams& p, const LoopParams
     }
     __syncwarp();
   }
+  // The limits, read before this block posts: block 0 rewrites them only after it
+  // has every block's word.  The streamed loop has them from the control
+  // block: with two more words of the clock the compiler gives its FP64 row loop
+  // other registers, 5 % slower (8192^2 1590 -> 1665 us a step).  In the resident
+  // loop the loads are 4 % (FP32 317x203 4.02 -> 4.18 us).
+  double t_stop;
+  long long most;
+  if constexpr (kState) {
+    t_stop = lp.more ? p.ctl->t_stop : lp.t_stop;
+    most = lp.more ? p.ctl->step_stop - p.ctl->step : lp.max_steps;
+  } else {
+    t_stop = ck.t_stop;
+    most = ck.most;
+  }
   // The new state, written by the whole block, before the word that says so.
   if (kState) __threadfence();
   post_max<M>(lp.slot, nb, buf, b, tag, bm);
   // Time and rain rate while the others' Hmax is on its way.
-  Clock& ck = S.clock;
   const double t = sc.t + sc.dt;
   double rate = 0.0;
   if (p.n_rain > 0) {
@@ -289,7 +321,7 @@ __device__ __forceinline__ void step_clock(const StepParams& p, const LoopParams
   const double dt_last = sc.dt;
   const bool bad = !(dt_last > 0.0) || !(t < 1.0e300) || !(hmax == hmax);
   const int status = !ok ? 2 : bad ? 1 : 0;
-  const bool done = status != 0 || !(t < lp.t_stop) || n + 1 >= lp.max_steps;
+  const bool done = status != 0 || !(t < t_stop) || n + 1 >= lp.slice || n + 1 >= most;
   __syncwarp();
   if (lane == 0) {
     if (!done) {
@@ -307,29 +339,34 @@ __device__ __forceinline__ void step_clock(const StepParams& p, const LoopParams
   }
 }
 
-// The control block after the loop (one thread of block 0), n steps on.
-template <typename T>
+// The control block after the launch (one thread of block 0), n steps on.
+template <typename T, typename N>
 __device__ inline void stop_clock(const StepParams& p, const LoopParams& lp,
-                                  const LoopShared<T>& S, int par0, unsigned tag0, long long n) {
+                                  const LoopShared<T>& S, int par0, unsigned tag0, N n) {
   SimCtl* ctl = p.ctl;
+  const Clock& k = S.clock;
   const long long limit = 0x3FFFFFFFFFFFFFFFLL;
-  ctl->t_stop = lp.t_stop;
-  ctl->step_stop = lp.max_steps > limit - ctl->step ? limit : ctl->step + lp.max_steps;
-  ctl->step += n;
-  ctl->done = 1;
+  if (!lp.more) {
+    ctl->t_stop = lp.t_stop;
+    ctl->step_stop = lp.max_steps > limit - ctl->step ? limit : ctl->step + lp.max_steps;
+  }
   ctl->arrive = 0u;
   if (n > 0) {
-    const Clock& k = S.clock;
+    ctl->step += n;
     ctl->t = k.t;
     ctl->hmax = k.hmax;
     ctl->dt_last = k.dt_last;
     ctl->rain_rate = k.rate;
     ctl->next_mass = k.next_mass;
     ctl->mass_count = k.mass_count;
-    ctl->parity = (par0 + (int)(n & 1)) & 1;
+    ctl->parity = par0 ^ (int)(n & 1);
     if (k.status != 0) atomicMax(&ctl->status, k.status);
     *lp.tag = tag0 + (unsigned)n + 16u;
   }
+  // A block that gave up in the last step may say so later than this; the next
+  // launch then takes no step and ends the call.
+  ctl->done = *(volatile int*)&ctl->status != 0 || !(ctl->t < ctl->t_stop) ||
+              ctl->step >= ctl->step_stop;
 }
 
 }  // namespace af

@@ -1,10 +1,10 @@
-// af_resident.cuh -- the time loop of a small grid in one launch, its state
-// held on chip.
+// af_resident.cuh -- the time loop of a small grid, many steps in one launch,
+// its state held on chip.
 //
 // A step of a small grid costs a kernel boundary, a prologue of dependent
 // loads and one trip to L2 per row, not bandwidth: 64 k cells took 11.4 us a
 // step and 0.8 M cells 20 us, against 0.3 and 3.4 us of HBM time.  Here one
-// cooperative launch runs all the steps of a call: block b of (at most) one
+// cooperative launch runs a call's steps (4 ms of them): block b of (at most) one
 // per SM keeps a band of rows in shared memory and exchanges with the others
 // only its first and last rows' new H and Qx and its Hmax.
 //
@@ -241,12 +241,9 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
 
   // ---- the loop's start, the same in every block
   const double t_start = ctl->t;
-  const int par0 = ctl->parity;
-  const unsigned tag0 = *rp.loop.tag;
-  long long n = 0;  // steps of this launch
-  const bool go = ctl->status == 0 && t_start < rp.loop.t_stop && rp.loop.max_steps > 0;
+  int n = 0;  // steps of this launch
   if (tid == 0) {
-    start_clock(p, S);
+    start_clock(p, rp.loop, S);
     // The band's marches: strip, first and last row.
     int q = 0;
     for (int gi = 0; gi < rp.gy; gi++) {
@@ -255,6 +252,7 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
     }
     s_nseg = q;
   }
+  __syncthreads();
   // The band's special cells and (consecutive, as cells are) their sources.
   const int e0 = rp.row_off[r0], ne = rp.row_off[r0 + nr] - e0;
   const int src0 = ne > 0 ? rp.row_spec[e0].s0 : 0;
@@ -267,7 +265,8 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
       if (q >= 0) s_bc[e] = boundary_depth<T>(p, q, at);
     }
   };
-  if (go) {
+  if (!S.done) {
+    const int par0 = S.par0;
     const T* gH = static_cast<const T*>(p.H[par0]);
     const T* gZ = static_cast<const T*>(p.DEM);
     const T* gX = static_cast<const T*>(p.Qx[par0]);
@@ -317,9 +316,9 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
   const int nseg = s_nseg;
   bool failed = false;
 #pragma unroll 1
-  while (go) {
-    const unsigned tag = tag0 + (unsigned)n;
-    const int buf = (int)(n & 1);
+  while (!S.done) {
+    const unsigned tag = S.tag0 + (unsigned)n;
+    const int buf = (n & 1);
     const StepScal<T>& sc = S.sc;  // warp 0 rewrites it past the march's barrier
     const T* const H = H0 + buf * nH;
     T* const Hn = H0 + (buf ^ 1) * nH;
@@ -484,14 +483,13 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
       failed = true;
       break;
     }
-    if (S.done) break;
   }
 
   // ---- the state back to its planes, and the control block
   if (failed && tid == 0) atomicExch(&ctl->status, 2);
-  const int par = (par0 + (int)(n & 1)) & 1;
+  const int par = S.par0 ^ (n & 1);
   if (!failed && n > 0) {
-    const int buf = (int)(n & 1);
+    const int buf = (n & 1);
     T* gH = static_cast<T*>(p.H[par]);
     T* gX = static_cast<T*>(p.Qx[par]);
     T* gY = static_cast<T*>(p.Qy[par]);
@@ -506,7 +504,7 @@ __global__ void __launch_bounds__(ResidentShape<T>::threads, 1)
       }
     }
   }
-  if (b == 0 && tid == 0) stop_clock(p, rp.loop, S, par0, tag0, n);
+  if (b == 0 && tid == 0) stop_clock(p, rp.loop, S, S.par0, S.tag0, n);
 }
 
 }  // namespace af

@@ -2,11 +2,12 @@
 // special-cell lists, and the launch that runs the time loop of one grid.
 // The padded field layout is described in af_simcore.cuh.
 //
-// The time loop (src/main.cpp:227 `while (t < sim_time)`) is one launch: a
-// cooperative kernel that holds the state on chip (af_resident.cuh) or streams
-// it from HBM (af_stream.cuh); where neither can be launched, a graph, in which
-// a begin kernel sets the stop condition, then a conditional WHILE node re-runs
-// the step kernel until its last block clears the condition.
+// The time loop (src/main.cpp:227 `while (t < sim_time)`) is a cooperative
+// kernel that holds the state on chip (af_resident.cuh) or streams it from HBM
+// (af_stream.cuh), launched again every few milliseconds by a conditional WHILE
+// node; where neither can be launched, a graph, in which a begin kernel sets the
+// stop condition, then a conditional WHILE node re-runs the step kernel until
+// its last block clears the condition.
 #include <algorithm>
 #include <cerrno>
 #include <cmath>
@@ -187,6 +188,11 @@ __global__ void k_begin(SimCtl* ctl, double t_stop, long long max_steps,
   if (use_cond) cudaGraphSetConditional(cond, done ? 0u : 1u);
 }
 
+// Whether the launch of the loop before this has left steps to another.
+__global__ void k_more(const SimCtl* ctl, cudaGraphConditionalHandle cond) {
+  cudaGraphSetConditional(cond, ctl->done ? 0u : 1u);
+}
+
 // Snapshot of the state for the file outputs: H and, when asked, the
 // velocity of ComputeVelocity_GPU (src/kernels.cpp:293-351), as dense FP64
 // fields in the reference layout.
@@ -254,8 +260,8 @@ struct Sim {
   DevBuf rain_times, rain_rates, spec_off, spec;
   DevBuf ctl, partials, mass_series, stage;
   size_t stage_bytes = 0;
-  // The whole loop in one cooperative launch of `loop_blocks` blocks: the state
-  // on chip (resident) or in HBM (stream); neither: the step kernel in a graph.
+  // Many steps in one cooperative launch of `loop_blocks` blocks: the state on
+  // chip (resident) or in HBM (stream); neither: the step kernel in a graph.
   bool resident = false, stream = false;
   DevBuf row_off, row_spec, exch;  // exch: slots, partials, tag and, resident, halos
   size_t exch_bytes = 0;
@@ -386,6 +392,14 @@ static bool can_loop(const void* fn, size_t need, int smem) {
          per_sm >= 1;
 }
 
+// Steps of one launch of the loop, of `us` each.  With a block per SM it keeps all
+// other work off the GPU until it ends (another simulation's loop, a batch, the
+// caller's own kernels), so it ends after kSliceUs.  A launch more costs some 20
+// us: us per step against one launch for the whole call FP32 317x203 3.97 / 3.95,
+// 2500x1801 29.4 / 29.3; FP64 1501x1100 47.7 / 47.5, 8192^2 1581 / 1581.
+constexpr double kSliceUs = 4000.0;
+static int slice_steps(double us) { return std::max(1, (int)(kSliceUs / us)); }
+
 // How the time loop runs (see Sim::resident).  AF_SIM_LOOP=resident, stream or
 // graph forces the choice (resident only where the state fits); host-driven
 // launches and a forced launch shape keep the step kernel.
@@ -417,8 +431,8 @@ static void pick_loop(Sim& s) {
     // 17.9 / 15.1.
     const double rows = resident_cost(s.c.nx, nr, kLoopWarps, gy);
     const double mcells = 1e-6 * s.c.nx * s.c.ny;
-    const bool faster = f64 ? 2.5 + 1.9 * rows < 11.0 + 14.0 * mcells
-                            : 2.4 + 0.6 * rows < 7.0 + 8.0 * mcells;
+    const double us = f64 ? 2.5 + 1.9 * rows : 2.4 + 0.6 * rows;
+    const bool faster = us < (f64 ? 11.0 + 14.0 * mcells : 7.0 + 8.0 * mcells);
     if ((faster || force) &&
         can_loop(f64 ? resident_kernel_f64() : resident_kernel_f32(), need, smem)) {
       s.resident = true;
@@ -426,6 +440,7 @@ static void pick_loop(Sim& s) {
       s.loop_smem = need;
       s.rprm.nr_max = nr;
       s.rprm.gy = gy;
+      s.rprm.loop.slice = slice_steps(us);
       return;
     }
   }
@@ -434,6 +449,10 @@ static void pick_loop(Sim& s) {
     s.stream = true;
     s.loop_blocks = (unsigned)sms;
     s.loop_smem = need;
+    // us per step: FP32 1024^2 13, 8192^2 326, 16384^2 1370; FP64 1501x1100 47,
+    // 8192^2 1587, 16384^2 6259.
+    const double mcells = 1e-6 * s.c.nx * s.c.ny;
+    s.rprm.loop.slice = slice_steps(f64 ? 11.0 + 23.5 * mcells : 7.0 + 5.0 * mcells);
   }
 }
 
@@ -587,6 +606,63 @@ static int setup_loop(Sim& s, std::vector<SpecCell> spec) {
     r.row_spec = (const SpecCell*)s.row_spec.p;
     // Pageable sources: wait until the copies have left host memory.
     AF_CUDA(cudaStreamSynchronize(s.st));
+  }
+  return AF_OK;
+}
+
+static const void* loop_fn(const Sim& s) {
+  const bool f64 = s.prec == AF_PREC_F64;
+  return s.resident ? (f64 ? resident_kernel_f64() : resident_kernel_f32())
+                    : (f64 ? stream_kernel_f64(s.tma) : stream_kernel_f32(s.tma));
+}
+
+// The graph of the launches after a call's first: while steps are left, the loop
+// again.  Where there cannot be one (cooperative kernels in it under MPS) the
+// simulation keeps the step kernel's.
+static int build_loop_graph(Sim& s) {
+  AF_CUDA(cudaGraphCreate(&s.graph, 0));
+  const SimCtl* ctl = s.prm.ctl;
+  ResidentParams r = s.rprm;
+  r.loop.more = 1;
+  bool ok = cudaGraphConditionalHandleCreate(&s.cond, s.graph, 0, 0) == cudaSuccess;
+  if (ok) {
+    void* margs[] = {&ctl, &s.cond};
+    cudaKernelNodeParams km{};
+    km.func = (void*)&k_more;
+    km.gridDim = dim3(1);
+    km.blockDim = dim3(1);
+    km.kernelParams = margs;
+    AF_CUDA(cudaGraphAddKernelNode(&s.begin_node, s.graph, nullptr, 0, &km));
+    cudaGraphNodeParams cp{};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = s.cond;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t cnode, lnode, mnode;
+    AF_CUDA(cudaGraphAddNode(&cnode, s.graph, &s.begin_node, 1, &cp));
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    void* rargs[] = {&s.prm, &r};
+    void* sargs[] = {&s.prm, &r.loop, &s.fields};
+    cudaKernelNodeParams kl{};
+    kl.func = const_cast<void*>(loop_fn(s));
+    kl.gridDim = dim3(s.loop_blocks);
+    kl.blockDim = dim3(32 * kLoopWarps);
+    kl.sharedMemBytes = (unsigned)s.loop_smem;
+    kl.kernelParams = s.resident ? rargs : sargs;
+    cudaKernelNodeAttrValue coop{};
+    coop.cooperative = 1;
+    ok = cudaGraphAddKernelNode(&lnode, body, nullptr, 0, &kl) == cudaSuccess &&
+         cudaGraphKernelNodeSetAttribute(lnode, cudaLaunchAttributeCooperative, &coop) ==
+             cudaSuccess &&
+         cudaGraphAddKernelNode(&mnode, body, &lnode, 1, &km) == cudaSuccess &&
+         cudaGraphInstantiate(&s.exec, s.graph, 0) == cudaSuccess;
+  }
+  if (!ok) {
+    cudaGetLastError();
+    cudaGraphDestroy(s.graph);
+    s.graph = nullptr;
+    s.exec = nullptr;
+    s.resident = s.stream = false;
   }
   return AF_OK;
 }
@@ -848,8 +924,11 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   p.mass_series = static_cast<double*>(s->mass_series.p);
   p.use_cond = 0;
   pick_loop(*s);
-  if (s->resident || s->stream) AF_TRY(setup_loop(*s, std::move(tb.spec)));
-  else AF_TRY(build_graph(*s));
+  if (s->resident || s->stream) {
+    AF_TRY(setup_loop(*s, std::move(tb.spec)));
+    AF_TRY(build_loop_graph(*s));
+  }
+  if (!s->resident && !s->stream) AF_TRY(build_graph(*s));
   AF_CUDA(cudaStreamSynchronize(s->st));
   *out = s.release();
   return AF_OK;
@@ -859,15 +938,15 @@ static int launch(Sim& s, double t_stop, long long max_steps) {
   AF_CUDA(cudaSetDevice(s.device));
   SimCtl* ctl = static_cast<SimCtl*>(s.ctl.p);
   if (s.resident || s.stream) {
-    const bool f64 = s.prec == AF_PREC_F64;
-    s.rprm.loop.t_stop = t_stop;
-    s.rprm.loop.max_steps = max_steps;
+    LoopParams& lp = s.rprm.loop;
+    lp.t_stop = t_stop;
+    lp.max_steps = max_steps;
+    lp.more = 0;
     void* rargs[] = {&s.prm, &s.rprm};
-    void* sargs[] = {&s.prm, &s.rprm.loop, &s.fields};
-    const void* fn = s.resident ? (f64 ? resident_kernel_f64() : resident_kernel_f32())
-                                : (f64 ? stream_kernel_f64(s.tma) : stream_kernel_f32(s.tma));
-    AF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(s.loop_blocks), dim3(32 * kLoopWarps),
+    void* sargs[] = {&s.prm, &lp, &s.fields};
+    AF_CUDA(cudaLaunchCooperativeKernel(loop_fn(s), dim3(s.loop_blocks), dim3(32 * kLoopWarps),
                                         s.resident ? rargs : sargs, s.loop_smem, s.st));
+    if (max_steps > lp.slice) AF_CUDA(cudaGraphLaunch(s.exec, s.st));
     return AF_OK;
   }
   if (s.use_cond) {

@@ -1,7 +1,7 @@
-// af_stream.cuh -- the time loop of a grid in HBM in one launch.
+// af_stream.cuh -- the time loop of a grid in HBM, many steps in one launch.
 //
-// The strips of af_step.cuh, one cooperative launch for all the steps of a
-// call: one block per SM, 16 warps, each marching its strips as k_step's
+// The strips of af_step.cuh, one cooperative launch for a call's steps, or as
+// many as take some 4 ms: one block per SM, 16 warps, each marching its strips as k_step's
 // one-warp blocks do, and between steps the exchange of af_exchange.cuh instead
 // of a kernel boundary.  A boundary costs its own launch, the last block's fold
 // (a chain of dependent loads and atomics, the rain look-up among them) and
@@ -44,8 +44,8 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
   const int par0 = ctl->parity;
   const unsigned tag0 = *lp.tag;
   long long n = 0;
-  const bool go = ctl->status == 0 && ctl->t < lp.t_stop && lp.max_steps > 0;
-  if (tid == 0) start_clock(p, S);
+  const bool go = loop_goes(ctl, lp);
+  if (tid == 0) start_clock(p, lp, S);
   uint64_t* const bar = s_bar[warp];
   if (lane == 0) {
     for (int s = 0; s < kStages; s++) mbar_init(&bar[s], 1);

@@ -1,8 +1,8 @@
 """Python host API over the simulation layer (af_sim_* in include/adaptflood.h).
 
 ``Simulation`` owns one device-resident case.  ``run(t_stop)`` is the
-reference's time loop ``while (t < sim_time)`` (src/main.cpp:227) as one
-launch; ``state()`` returns full-precision fields in the
+reference's time loop ``while (t < sim_time)`` (src/main.cpp:227), enqueued by
+one call; ``state()`` returns full-precision fields in the
 reference's layout; ``velocity()`` is ComputeVelocity_GPU
 (src/kernels.cpp:293-351) on the device.  ``load_par()`` reads a case from
 ``.par`` files with the reference's parsing rules.

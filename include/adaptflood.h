@@ -15,7 +15,7 @@
  *    ends in Kokkos::fence().  The reference's functions return void and abort
  *    on error; these return AF_OK or a negative AF_E* code.
  *
- * 2. The simulation layer (af_sim_*): the whole time loop in one launch of
+ * 2. The simulation layer (af_sim_*): the time loop in launches of many
  *    fused steps with device-resident dt, time and hydrograph interpolation, in
  *    FP64 (results within 1e-9 m of the reference) or FP32 state with FP64
  *    time, interpolation and volume accumulation.
@@ -209,7 +209,9 @@ int af_sim_create(const af_case_desc* c, const af_forcing_desc* f, const double*
 int af_sim_destroy(af_sim* s);
 
 /* Enqueues steps while t < t_stop and fewer than max_steps steps have run in
- * this call (the loop test of src/main.cpp:227), without waiting. */
+ * this call (the loop test of src/main.cpp:227), without waiting.  The steps
+ * take the whole GPU for some milliseconds at a time; work on other streams (another
+ * simulation, a batch, the caller's kernels) runs in between. */
 int af_sim_launch(af_sim* s, double t_stop, int64_t max_steps);
 /* Waits for the enqueued steps. */
 int af_sim_sync(af_sim* s);
