@@ -258,8 +258,7 @@ struct Sim {
   DevBuf src_type, src_value, src_off, src_times, src_vals, src_sorted;
   DevBuf bc_type, bc_value, bc_off, bc_times, bc_vals, bc_sorted;
   DevBuf rain_times, rain_rates, spec_off, spec;
-  DevBuf ctl, partials, mass_series, stage;
-  size_t stage_bytes = 0;
+  DevBuf ctl, partials, mass_series;
   // Many steps in one cooperative launch of `loop_blocks` blocks: the state on
   // chip (resident) or in HBM (stream); neither: the step kernel in a graph.
   bool resident = false, stream = false;
@@ -473,45 +472,39 @@ static int alloc_field(DevBuf& b, size_t elems, int esize) {
 }
 
 // Field transfers between the caller's FP64 host arrays (rows of `width`
-// values at host pitch `hpitch`) and a padded device field, through the
-// simulation's staging buffer (made on first use and kept: a field, at most
-// kStageBytes, less where the device has no more; none for long FP64 rows).
-static int get_stage(Sim& s) {
-  const bool f64 = s.prec == AF_PREC_F64;
-  if (s.stage.p || (f64 && (size_t)s.c.nx * 8 >= kLongRow)) return AF_OK;
-  size_t want = std::min(kStageBytes, (size_t)(s.c.ny + 1) * (s.c.nx + 1) * 8);
-  for (;; want /= 8) {
-    if (cudaMalloc(&s.stage.p, want) == cudaSuccess) break;
-    const cudaError_t e = cudaGetLastError();
-    s.stage.p = nullptr;
-    if (want < (64u << 10)) {
-      if (f64) return AF_OK;  // the direct copy
-      cuda_fail(e);
-      return AF_ENOMEM;
-    }
-  }
-  s.stage_bytes = want;
+// values at host pitch `hpitch`) and a padded device field, through Qx and Qy of
+// the parity that does not hold the state: nothing there is read before the next
+// step writes it, except the padding, so it is left zero.
+static double* stage_of(Sim& s, int par, size_t& cap) {
+  cap = std::min(kStageBytes, 2 * s.qy_elems * s.esize / 8 * 8);
+  return static_cast<double*>(s.Qx[par ^ 1].p);
+}
+static int clear_stage(Sim& s, double* stage, size_t cap, int rows, int width) {
+  if (s.prec == AF_PREC_F64 && direct_rows(width)) return AF_OK;
+  AF_CUDA(cudaMemsetAsync(stage, 0, std::min(cap, (size_t)rows * width * 8), s.st));
   return AF_OK;
 }
 
-static int put_field(Sim& s, DevBuf& b, const double* src, int rows, int width, size_t hpitch) {
-  AF_TRY(get_stage(s));
-  double* const stage = static_cast<double*>(s.stage.p);
-  const size_t cap = s.stage_bytes;
+static int put_field(Sim& s, int par, DevBuf& b, const double* src, int rows, int width,
+                     size_t hpitch) {
+  size_t cap;
+  double* const stage = stage_of(s, par, cap);
   AF_TRY(s.prec == AF_PREC_F64
              ? put_rows(s.buf<double>(b), s.P, src, rows, width, hpitch, stage, cap, s.st)
              : put_rows(s.buf<float>(b), s.P, src, rows, width, hpitch, stage, cap, s.st));
+  AF_TRY(clear_stage(s, stage, cap, rows, width));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }
 
-static int get_field(Sim& s, DevBuf& b, double* dst, int rows, int width, size_t hpitch) {
-  AF_TRY(get_stage(s));
-  double* const stage = static_cast<double*>(s.stage.p);
-  const size_t cap = s.stage_bytes;
+static int get_field(Sim& s, int par, DevBuf& b, double* dst, int rows, int width,
+                     size_t hpitch) {
+  size_t cap;
+  double* const stage = stage_of(s, par, cap);
   AF_TRY(s.prec == AF_PREC_F64
              ? get_rows(s.buf<double>(b), s.P, dst, rows, width, hpitch, stage, cap, s.st)
              : get_rows(s.buf<float>(b), s.P, dst, rows, width, hpitch, stage, cap, s.st));
+  AF_TRY(clear_stage(s, stage, cap, rows, width));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }
@@ -826,9 +819,9 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
     order[k]->p = static_cast<char*>(s->planes.p) + k * plane_bytes;
     order[k]->own = false;
   }
-  AF_TRY(put_field(*s, s->DEM, dem, ny, nx, nx));
+  AF_TRY(put_field(*s, 0, s->DEM, dem, ny, nx, nx));
   AF_CUDA(cudaMemcpyAsync(s->DEM2.p, s->DEM.p, plane_bytes, cudaMemcpyDeviceToDevice, s->st));
-  if (h0) AF_TRY(put_field(*s, s->H[0], h0, ny, nx, nx));
+  if (h0) AF_TRY(put_field(*s, 0, s->H[0], h0, ny, nx, nx));
   AF_TRY(encode_fields(*s));
 
   HostTables tb;
@@ -925,8 +918,14 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   p.use_cond = 0;
   pick_loop(*s);
   if (s->resident || s->stream) {
-    AF_TRY(setup_loop(*s, std::move(tb.spec)));
-    AF_TRY(build_loop_graph(*s));
+    const int rc = setup_loop(*s, std::move(tb.spec));
+    if (rc == AF_ENOMEM) {  // the step kernel needs no exchange
+      cudaGetLastError();
+      s->resident = s->stream = false;
+    } else {
+      AF_TRY(rc);
+      AF_TRY(build_loop_graph(*s));
+    }
   }
   if (!s->resident && !s->stream) AF_TRY(build_graph(*s));
   AF_CUDA(cudaStreamSynchronize(s->st));
@@ -1050,13 +1049,13 @@ int af_sim_get_state(af_sim* h, double* H, double* Qx, double* Qy) {
   AF_TRY(af::read_ctl(s));
   const int par = s.pinned_ctl->parity;
   const int nx = s.c.nx, ny = s.c.ny;
-  if (H) AF_TRY(af::get_field(s, s.H[par], H, ny, nx, nx));
+  if (H) AF_TRY(af::get_field(s, par, s.H[par], H, ny, nx, nx));
   if (Qx) {
-    AF_TRY(af::get_field(s, s.Qx[par], Qx, ny, nx + 1, nx + 1));
+    AF_TRY(af::get_field(s, par, s.Qx[par], Qx, ny, nx + 1, nx + 1));
     for (int i = 0; i <= nx; i++) Qx[(size_t)ny * (nx + 1) + i] = 0.0;
   }
   if (Qy) {
-    AF_TRY(af::get_field(s, s.Qy[par], Qy, ny + 1, nx, nx + 1));
+    AF_TRY(af::get_field(s, par, s.Qy[par], Qy, ny + 1, nx, nx + 1));
     for (int j = 0; j <= ny; j++) Qy[(size_t)j * (nx + 1) + nx] = 0.0;
   }
   return AF_OK;
@@ -1069,9 +1068,9 @@ int af_sim_set_state(af_sim* h, const double* H, const double* Qx, const double*
   AF_TRY(af::read_ctl(s));
   const int par = s.pinned_ctl->parity;
   const int nx = s.c.nx, ny = s.c.ny;
-  if (H) AF_TRY(af::put_field(s, s.H[par], H, ny, nx, nx));
-  if (Qx) AF_TRY(af::put_field(s, s.Qx[par], Qx, ny, nx + 1, nx + 1));
-  if (Qy) AF_TRY(af::put_field(s, s.Qy[par], Qy, ny + 1, nx, nx + 1));
+  if (H) AF_TRY(af::put_field(s, par, s.H[par], H, ny, nx, nx));
+  if (Qx) AF_TRY(af::put_field(s, par, s.Qx[par], Qx, ny, nx + 1, nx + 1));
+  if (Qy) AF_TRY(af::put_field(s, par, s.Qy[par], Qy, ny + 1, nx, nx + 1));
   af::SimCtl& c = *s.pinned_ctl;
   c.t = t;
   c.rain_rate = s.n_rain > 0 ? af::interp_series(s.rain_t.data(), s.rain_r.data(), s.n_rain, 0.0,

@@ -188,6 +188,7 @@ __global__ void k_volume_int(const T* __restrict__ H, int nx, int ny, int P, dou
 constexpr size_t kStageBytes = 64u << 20;
 // FP64 rows at least this long go straight into the padded field.
 constexpr size_t kLongRow = 16384;
+inline bool direct_rows(int width) { return (size_t)width * 8 >= kLongRow; }
 
 template <typename T>
 __global__ void k_pad_from_f64(const double* __restrict__ src, int rows, int width,
@@ -211,12 +212,11 @@ __global__ void k_dense_to_f64(const T* __restrict__ src, int P, int rows, int w
 }
 
 // Caller FP64 rows at host pitch `hpitch` -> a padded device field at `dst`, and
-// back, through the `cap` bytes of `stage` (FP64: null takes the direct copy).
-// A row longer than that goes in parts.
+// back, through the `cap` bytes of `stage`.  A row longer than that goes in parts.
 template <typename T>
 int put_rows(T* dst, int P, const double* src, int rows, int width, size_t hpitch, double* stage,
              size_t cap, cudaStream_t st) {
-  if (sizeof(T) == 8 && (!stage || (size_t)width * 8 >= kLongRow)) {
+  if (sizeof(T) == 8 && direct_rows(width)) {
     AF_CUDA(copy2d_h2d(dst, (size_t)P * 8, src, hpitch * 8, (size_t)width * 8, rows, st));
     return AF_OK;
   }
@@ -238,7 +238,7 @@ int put_rows(T* dst, int P, const double* src, int rows, int width, size_t hpitc
 template <typename T>
 int get_rows(const T* src, int P, double* dst, int rows, int width, size_t hpitch, double* stage,
              size_t cap, cudaStream_t st) {
-  if (sizeof(T) == 8 && (!stage || (size_t)width * 8 >= kLongRow)) {
+  if (sizeof(T) == 8 && direct_rows(width)) {
     AF_CUDA(copy2d_d2h(dst, hpitch * 8, src, (size_t)P * 8, (size_t)width * 8, rows, st));
     return AF_OK;
   }
