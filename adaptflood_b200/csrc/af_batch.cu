@@ -64,6 +64,7 @@ static size_t align_up(size_t x) { return (x + Arena::kAlign - 1) / Arena::kAlig
 // Byte offsets of one scenario's arrays inside its arena block.
 struct Layout {
   int nx = 0, ny = 0, P = 0, R = 0, nsx = 0, nsy = 0;
+  int rmin = 1;  // the lowest strips that the per-strip arrays hold
   size_t H[2], Qx[2], Qy[2], DEM;
   size_t src_type, src_value, src_off, src_times, src_vals, src_sorted;
   size_t bc_type, bc_value, bc_off, bc_times, bc_vals, bc_sorted;
@@ -86,9 +87,17 @@ static Layout make_layout(const af_case_desc* c, const af_forcing_desc* f, doubl
   L.nx = c->nx;
   L.ny = c->ny;
   L.P = row_pitch(c->nx, N);
-  L.R = R;
   L.nsx = strips_x(c->nx, N);
-  L.nsy = (c->ny + R - 1) / R;
+  // Per-strip arrays are sized for the lowest strips, so the strip height can
+  // change between launches without moving anything.  Those are of one row in
+  // FP32, and in FP64, whose strips are half as wide (30 columns), of as many as
+  // a 16-byte lane's strips of one row are worth: one-row strips would take 0.8 %
+  // more of the arena, so that fewer grids fit.
+  const size_t nstrips =
+      std::max((size_t)L.nsx, (size_t)strips_x(c->nx, 16 / esize) * (size_t)c->ny);
+  while ((size_t)L.nsx * ((c->ny + L.rmin - 1) / L.rmin) > nstrips) L.rmin++;
+  L.R = std::max(R, L.rmin);
+  L.nsy = (c->ny + L.R - 1) / L.R;
   size_t at = 0;
   auto put = [&](size_t bytes) {
     const size_t o = at;
@@ -119,9 +128,6 @@ static Layout make_layout(const af_case_desc* c, const af_forcing_desc* f, doubl
   L.bc_sorted = put(no);
   L.rain_times = put(sizeof(double) * f->n_rain);
   L.rain_rates = put(sizeof(double) * f->n_rain);
-  // Per-strip arrays are sized for one-row strips, so the strip height can
-  // change between launches without moving anything.
-  const size_t nstrips = (size_t)L.nsx * L.ny;
   L.spec_off = put(sizeof(int) * (nstrips + 1));
   L.spec = put(sizeof(SpecCell) * (size_t)(nf + no));  // at most one per source or BC
   L.partials = put(sizeof(double) * 3 * nstrips);
@@ -378,7 +384,7 @@ static int add(Batch& b, const af_case_desc* c, const af_forcing_desc* f, const 
     return rc;
   };
   HostTables tb;
-  build_tables(c, f, 30 * b.N, R, L.nsx, L.nsy, tb);
+  build_tables(c, f, 30 * b.N, L.R, L.nsx, L.nsy, tb);
   char* base = b.arena + off;
   int rc = AF_OK;
   if (cudaMemsetAsync(base, 0, L.total, b.cst) != cudaSuccess)
@@ -550,11 +556,12 @@ static int set_slot_rows(Batch& b, int slot, int R) {
   return AF_OK;
 }
 
-// Strips of the active members with heights of at most R (and of the heights
-// that the caller set).
+// A member's strip height for heights of at most R (and of the height that the
+// caller set).
 static int height_of(const Batch& b, int slot, int R) {
   const int cls = b.slots[slot].cls;
-  return b.balance == kAuto && !b.rows_set[cls] ? R : std::max(1, std::min(b.rows[cls], R));
+  const int r = b.balance == kAuto && !b.rows_set[cls] ? R : std::min(b.rows[cls], R);
+  return std::max(b.slots[slot].L.rmin, r);
 }
 static long long strips_of(const Batch& b, const std::vector<int>& act, int R) {
   long long u = 0;
