@@ -606,12 +606,14 @@ static int retile(Batch& b) {
     }
     int tall = 0;
     long long now = 0;
+    bool kept = true;  // the heights that the caller has set since
     for (int k : act) {
       const Layout& L = b.slots[k].L;
       tall = std::max(tall, L.R);
       now += (long long)L.nsx * L.nsy;
+      kept = kept && height_of(b, k, L.R) == L.R;
     }
-    if (step_rows(now, tall, W) <= 1.03 * best) return AF_OK;
+    if (kept && step_rows(now, tall, W) <= 1.03 * best) return AF_OK;
   } else {
     for (int R = 4096; R >= 2; R >>= 1)
       if (strips_of(b, act, R) >= b.balance * W) {
