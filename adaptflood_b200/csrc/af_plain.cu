@@ -743,7 +743,9 @@ int af_floodplain_q(const double* H, const double* DEM, double* Qx, double* Qy,
   if (theta == 1.0) {
     const double dxinv = 1.0 / dx;
     const bool in_range = face_range_ok(dx, FPn, DepthThresh, MaxHflow, 1.0);
-    const dim3 gq((xsz + 31) / 32, (ysz + 7) / 8);
+    // One column has no face in its last row (its grid is as tall as k_qy's).
+    const int rows = xsz > 1 ? ysz : std::max(1, ysz - 1);
+    const dim3 gq((xsz + 31) / 32, (rows + 7) / 8);
     k_faces<<<gq, 256, 0, st>>>(H, DEM, Qx, Qy, Qxold, Qyold, xsz, ysz, dx, dxinv,
                                 std::fma(-dx, dxinv, 1.0) / dx, FPn, DepthThresh, MaxHflow, out, g,
                                 nodata, in_range);
