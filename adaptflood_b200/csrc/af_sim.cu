@@ -296,6 +296,8 @@ static const void* step_fn(const Sim& s) {
                                : step_kernel_f32(s.variant, s.tma);
 }
 
+static void pick_loop(Sim& s);
+
 static int pick_shape(Sim& s) {
   const int own = 30 * s.N;
   s.nsx = (s.c.nx + own - 1) / own;
@@ -318,34 +320,41 @@ static int pick_shape(Sim& s) {
     per_sm = 1;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long slots = (long long)sms * per_sm;  // resident blocks
+  pick_loop(s);
+  // Strips (k_step: blocks of strips) that run at a time.
+  const long long slots = (long long)sms * (s.stream ? kLoopWarps : per_sm);
+  const int wy = s.stream ? 1 : s.WY;
   auto tiles_for = [&](int R) {
     const long long nsy = (s.c.ny + R - 1) / R;
-    return (long long)s.nsx * ((nsy + s.WY - 1) / s.WY);
+    return (long long)s.nsx * ((nsy + wy - 1) / wy);
   };
   // Rows per strip: the height that gives the busiest warp the fewest rows, each
   // strip counted with 1.2 rows more for its first loads and faces, up to a
-  // limit.  us per step at that height and at others: FP32 1400^2 R8 16.4,
-  // 2500x1801 R17 30.6 (R8 30.3, R12 33.8, R32 39.9), 3072^2 R17 54 (R8 57, R32
-  // 72); FP64 700^2 R8 20.6 (R4 21.8, R16 26.5), 1501x1100 R24 47.4 (R8 50.5, R32
-  // 53.0), 2731x2747 R18 191 (R8 208, R16 195), 4096^2 R32 414 (R16 417).
-  // The FP32 limit is the L2's: strips side by side share the cache lines at
+  // limit.  us per step of the streamed loop at that height and at others: FP32
+  // 2000x220 R2 8.7 (R1 9.8, R4 9.5), 6000x170 R4 11.2 (R1 14.9, R2 11.7), 1000^2
+  // R4 10.9 (R1 15.3, R2 12.4), 2500x1801 R17 30.6 (R8 30.3, R12 33.8, R32 39.9),
+  // 3072^2 R17 54 (R8 57, R32 72); FP64 700^2 R8 20.6 (R4 21.8, R16 26.5), 1501x1100
+  // R24 47.4 (R8 50.5, R32 53.0), 2731x2747 R18 191 (R8 208, R16 195), 4096^2 R32 414
+  // (R16 417).
+  // The FP32 limits are fitted.  Strips side by side share the cache lines at
   // their edges and strips one above the other a row, read from DRAM once only
   // while what all warps work on at a time (their number x R rows x 120 columns x
-  // 28 bytes) stays in the 126 MB, with room for warps that are ahead: 5792^2 R10
-  // 168, R12 167, R14 175, R32 194; 8192^2 R6 338, R8 326, R10 328, R12 352,
-  // R32 388; 16384^2 R6 1380, R7 1370, R8 1380, R10 1460, R32 1630, mostly dry
-  // R6 1304, R7 1292, R8 1395, R32 1616.  Up to 2^23 cells taller strips cost
-  // nothing.
+  // 28 bytes, 8 MB a row) stays in the 126 MB of L2, with room for warps that are
+  // ahead; that alone would allow some 12 rows at every size, but the best height
+  // falls further as grids grow, for a reason that is not established: 5792^2 R10
+  // 172, R12 169, R14 174, R16 182, R32 198; 8192^2 R6 338, R8 331, R10 331, R12 341,
+  // R16 369, R32 392; 10000x9000 R6 464, R8 432, R10 449, R12 482, R32 546; 16384^2 R6
+  // 1380, R7 1370, R8 1380, R10 1460, R32 1630, mostly dry R6 1304, R7 1292, R8 1395,
+  // R32 1616.  Taller strips cost little up to 2^23 cells (2900^2 R16 49.9, R32 51.7).
   // FP64 is bound by its arithmetic (16384^2 R32 6259, R16 6457, R8 6928).
   const long long cells = (long long)s.c.nx * s.c.ny;
   const bool f64 = s.prec == AF_PREC_F64;
   s.R = 32;
-  if (!f64 && cells < (1LL << 20)) {
-    // Small FP32 grids: one-row strips, the shortest chain per warp even at
-    // slightly over one wave (ms per step in a graph of step kernels, one row
-    // against the shortest strips that fit in one wave: 512^2 0.0312 / 0.0369,
-    // 724^2 0.0372 / 0.0393; at 1024^2 and above the rule is as fast or faster).
+  if (!f64 && !s.stream && cells < (1LL << 20)) {
+    // Small FP32 grids in the graph of step kernels: one-row strips, the shortest
+    // chain per warp even at slightly over one wave (ms per step, one row against
+    // the shortest strips that fit in one wave: 512^2 0.0312 / 0.0369, 724^2 0.0372 /
+    // 0.0393; at 1024^2 and above the rule is as fast or faster).
     s.R = 1;
   } else if (!f64 || cells <= (1LL << 24)) {
     const int lo = f64 ? 4 : 2;
@@ -369,7 +378,7 @@ static int pick_shape(Sim& s) {
   // Persistent grid: as many blocks as fit on the GPU at once (a whole number
   // of blocks per SM), never more than there are tiles.
   const long long tiles = (long long)s.nsx * ((s.nsy + s.WY - 1) / s.WY);
-  s.grid = dim3((unsigned)(tiles < slots ? tiles : slots));
+  s.grid = dim3((unsigned)std::min(tiles, (long long)sms * per_sm));
   s.block = dim3(32 * s.WY);
   return AF_OK;
 }
@@ -425,9 +434,11 @@ static void pick_loop(Sim& s) {
     // (12 of 16 us on an FP64 grid 640 wide, whose 20 strips take 16 warps two
     // rounds), the streamed one with the cells.  Estimated us per step, fitted
     // to 128^2 ... 1023x769 FP32 and 128^2 ... 700^2 FP64; measured resident /
-    // streamed: FP32 317x203 4.2 / 7.4, 512^2 5.4 / 8.8, 1023x769 10.2 / 13.3,
-    // 2000x220 10.9 / 9.8; FP64 317x203 7.6 / 11.7, 512^2 13.3 / 13.9, 640x512
-    // 17.9 / 15.1.
+    // streamed: FP32 317x203 4.0 / 7.5, 512^2 5.0 / 8.1, 724^2 7.4 / 10.0, 900^2
+    // 10.2 / 12.0, 2000x220 10.9 / 8.5, 1200x500 10.7 / 9.9, 2900x100 12.1 / 8.0;
+    // FP64 317x203 7.6 / 11.7, 512^2 13.3 / 13.9, 640x512 17.9 / 15.1.  Near the
+    // line it may take the other one, by 9 % at most where measured (1023x769
+    // takes 10.2 / 9.7, 1500x300 9.1 / 8.5 and streams 700x1200, 10.0 / 10.9).
     const double rows = resident_cost(s.c.nx, nr, kLoopWarps, gy);
     const double mcells = 1e-6 * s.c.nx * s.c.ny;
     const double us = f64 ? 2.5 + 1.9 * rows : 2.4 + 0.6 * rows;
@@ -916,7 +927,6 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   p.partials = static_cast<double*>(s->partials.p);
   p.mass_series = static_cast<double*>(s->mass_series.p);
   p.use_cond = 0;
-  pick_loop(*s);
   if (s->resident || s->stream) {
     const int rc = setup_loop(*s, std::move(tb.spec));
     if (rc == AF_ENOMEM) {  // the step kernel needs no exchange
