@@ -247,13 +247,14 @@ __device__ __forceinline__ void step_clock(const StepParams& p, const LoopParams
     __syncwarp();
   }
   // The limits, read before this block posts: block 0 rewrites them only after it
-  // has every block's word.  The streamed loop has them from the control
-  // block: with two more words of the clock the compiler gives its FP64 row loop
-  // other registers, 5 % slower (8192^2 1590 -> 1665 us a step).  In the resident
-  // loop the loads are 4 % (FP32 317x203 4.02 -> 4.18 us).
+  // has every block's word.  The streamed FP64 loop has them from the control
+  // block: with two more words of the clock the compiler gives its row loop other
+  // registers, 5 % slower (8192^2 1590 -> 1665 us a step).  In the other loops the
+  // loads cost (resident FP32 317x203 4.02 -> 4.18 us, streamed 2500x1801 31.2 ->
+  // 31.4).
   double t_stop;
   long long most;
-  if constexpr (kState) {
+  if constexpr (kState && sizeof(T) == 8) {
     t_stop = lp.more ? p.ctl->t_stop : lp.t_stop;
     most = lp.more ? p.ctl->step_stop - p.ctl->step : lp.max_steps;
   } else {

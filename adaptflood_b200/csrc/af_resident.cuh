@@ -4,7 +4,7 @@
 // A step of a small grid costs a kernel boundary, a prologue of dependent
 // loads and one trip to L2 per row, not bandwidth: 64 k cells took 11.4 us a
 // step and 0.8 M cells 20 us, against 0.3 and 3.4 us of HBM time.  Here one
-// cooperative launch runs a call's steps (4 ms of them): block b of (at most) one
+// cooperative launch runs a call's steps (8 ms of them): block b of (at most) one
 // per SM keeps a band of rows in shared memory and exchanges with the others
 // only its first and last rows' new H and Qx and its Hmax.
 //

@@ -4,8 +4,8 @@
 //
 // The time loop (src/main.cpp:227 `while (t < sim_time)`) is a cooperative
 // kernel that holds the state on chip (af_resident.cuh) or streams it from HBM
-// (af_stream.cuh), launched again every few milliseconds by a conditional WHILE
-// node; where neither can be launched, a graph, in which a begin kernel sets the
+// (af_stream.cuh), launched again every few milliseconds, by the host or by a
+// conditional WHILE node; where neither can be launched, a graph, in which a begin kernel sets the
 // stop condition, then a conditional WHILE node re-runs the step kernel until
 // its last block clears the condition.
 #include <algorithm>
@@ -275,6 +275,7 @@ struct Sim {
   cudaGraphNode_t begin_node = nullptr;
   cudaGraphConditionalHandle cond = 0;
   bool use_cond = false;
+  bool graph_tried = false;
   int n_rain = 0;
   std::vector<double> rain_t, rain_r;
   uint64_t case_hash = 0;  // case parameters and forcing (checkpoint identity)
@@ -402,10 +403,11 @@ static bool can_loop(const void* fn, size_t need, int smem) {
 
 // Steps of one launch of the loop, of `us` each.  With a block per SM it keeps all
 // other work off the GPU until it ends (another simulation's loop, a batch, the
-// caller's own kernels), so it ends after kSliceUs.  A launch more costs some 20
-// us: us per step against one launch for the whole call FP32 317x203 3.97 / 3.95,
-// 2500x1801 29.4 / 29.3; FP64 1501x1100 47.7 / 47.5, 8192^2 1581 / 1581.
-constexpr double kSliceUs = 4000.0;
+// caller's own kernels), so it ends after kSliceUs.  A launch more costs 20 to
+// 40 us (the gap, the first step's loads): us per step in launches of 8 ms against
+// one for the whole call FP32 317x203 3.97 / 3.95, 2500x1801 29.2 / 29.3; FP64
+// 1501x1100 47.4 / 47.4, 2731x2747 187.4 / 187.4.
+constexpr double kSliceUs = 8000.0;
 static int slice_steps(double us) { return std::max(1, (int)(kSliceUs / us)); }
 
 // How the time loop runs (see Sim::resident).  AF_SIM_LOOP=resident, stream or
@@ -620,15 +622,47 @@ static const void* loop_fn(const Sim& s) {
                     : (f64 ? stream_kernel_f64(s.tma) : stream_kernel_f32(s.tma));
 }
 
-// The graph of the launches after a call's first: while steps are left, the loop
-// again.  Where there cannot be one (cooperative kernels in it under MPS) the
-// simulation keeps the step kernel's.
-static int build_loop_graph(Sim& s) {
-  AF_CUDA(cudaGraphCreate(&s.graph, 0));
+// One launch of the loop: the call's first, or (more) one that goes on with it.
+static int launch_slice(Sim& s, int more) {
+  s.rprm.loop.more = more;
+  void* rargs[] = {&s.prm, &s.rprm};
+  void* sargs[] = {&s.prm, &s.rprm.loop, &s.fields};
+  AF_CUDA(cudaLaunchCooperativeKernel(loop_fn(s), dim3(s.loop_blocks), dim3(32 * kLoopWarps),
+                                      s.resident ? rargs : sargs, s.loop_smem, s.st));
+  return AF_OK;
+}
+
+// Launches of the loop that a call of `steps` steps takes.
+static long long slices_of(const Sim& s, double steps) {
+  const double n = std::ceil(steps / s.rprm.loop.slice);
+  return n >= 1e15 ? (long long)1e15 : n >= 1.0 ? (long long)n : 1;  // NaN: 1
+}
+constexpr long long kMaxQueued = 16;  // launches enqueued one by one
+
+// A call's launches after its first, as many at a time as its last dt lets it
+// expect, until it is done.
+static int finish_slices(Sim& s) {
+  for (;;) {
+    AF_TRY(read_ctl(s));
+    const SimCtl& c = *s.pinned_ctl;
+    if (c.done) return AF_OK;
+    const double left =
+        std::min((c.t_stop - c.t) / c.dt_last, (double)(c.step_stop - c.step));
+    for (long long n = std::min(kMaxQueued, slices_of(s, left)); n > 0; n--)
+      AF_TRY(launch_slice(s, 1));
+  }
+}
+
+// The graph that launches the loop again while steps are left, for calls of many
+// launches that must not wait; made when first needed (0.5 ms).
+static bool loop_graph(Sim& s) {
+  if (s.exec || s.graph_tried) return s.exec != nullptr;
+  s.graph_tried = true;
   const SimCtl* ctl = s.prm.ctl;
   ResidentParams r = s.rprm;
   r.loop.more = 1;
-  bool ok = cudaGraphConditionalHandleCreate(&s.cond, s.graph, 0, 0) == cudaSuccess;
+  bool ok = cudaGraphCreate(&s.graph, 0) == cudaSuccess &&
+            cudaGraphConditionalHandleCreate(&s.cond, s.graph, 0, 0) == cudaSuccess;
   if (ok) {
     void* margs[] = {&ctl, &s.cond};
     cudaKernelNodeParams km{};
@@ -636,15 +670,6 @@ static int build_loop_graph(Sim& s) {
     km.gridDim = dim3(1);
     km.blockDim = dim3(1);
     km.kernelParams = margs;
-    AF_CUDA(cudaGraphAddKernelNode(&s.begin_node, s.graph, nullptr, 0, &km));
-    cudaGraphNodeParams cp{};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = s.cond;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode, lnode, mnode;
-    AF_CUDA(cudaGraphAddNode(&cnode, s.graph, &s.begin_node, 1, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
     void* rargs[] = {&s.prm, &r};
     void* sargs[] = {&s.prm, &r.loop, &s.fields};
     cudaKernelNodeParams kl{};
@@ -655,20 +680,26 @@ static int build_loop_graph(Sim& s) {
     kl.kernelParams = s.resident ? rargs : sargs;
     cudaKernelNodeAttrValue coop{};
     coop.cooperative = 1;
-    ok = cudaGraphAddKernelNode(&lnode, body, nullptr, 0, &kl) == cudaSuccess &&
+    cudaGraphNodeParams cp{};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = s.cond;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t cnode, lnode, mnode;
+    ok = cudaGraphAddKernelNode(&s.begin_node, s.graph, nullptr, 0, &km) == cudaSuccess &&
+         cudaGraphAddNode(&cnode, s.graph, &s.begin_node, 1, &cp) == cudaSuccess;
+    cudaGraph_t body = ok ? cp.conditional.phGraph_out[0] : nullptr;
+    ok = ok && cudaGraphAddKernelNode(&lnode, body, nullptr, 0, &kl) == cudaSuccess &&
          cudaGraphKernelNodeSetAttribute(lnode, cudaLaunchAttributeCooperative, &coop) ==
              cudaSuccess &&
          cudaGraphAddKernelNode(&mnode, body, &lnode, 1, &km) == cudaSuccess &&
          cudaGraphInstantiate(&s.exec, s.graph, 0) == cudaSuccess;
   }
-  if (!ok) {
+  if (!ok) {  // under MPS, for one: cooperative kernels cannot be in such a graph
     cudaGetLastError();
-    cudaGraphDestroy(s.graph);
-    s.graph = nullptr;
     s.exec = nullptr;
-    s.resident = s.stream = false;
   }
-  return AF_OK;
+  return ok;
 }
 
 static int build_graph(Sim& s) {
@@ -934,7 +965,6 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
       s->resident = s->stream = false;
     } else {
       AF_TRY(rc);
-      AF_TRY(build_loop_graph(*s));
     }
   }
   if (!s->resident && !s->stream) AF_TRY(build_graph(*s));
@@ -943,19 +973,24 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   return AF_OK;
 }
 
-static int launch(Sim& s, double t_stop, long long max_steps) {
+// Enqueues a call's steps; where `wait` is allowed it may wait for them.  A call of
+// many launches that must not wait leaves all but the first to the graph, whose end
+// costs some 50 us; a call that waits makes its launches as it sees how far it is.
+static int launch(Sim& s, double t_stop, long long max_steps, bool wait = false) {
   AF_CUDA(cudaSetDevice(s.device));
   SimCtl* ctl = static_cast<SimCtl*>(s.ctl.p);
   if (s.resident || s.stream) {
-    LoopParams& lp = s.rprm.loop;
-    lp.t_stop = t_stop;
-    lp.max_steps = max_steps;
-    lp.more = 0;
-    void* rargs[] = {&s.prm, &s.rprm};
-    void* sargs[] = {&s.prm, &lp, &s.fields};
-    AF_CUDA(cudaLaunchCooperativeKernel(loop_fn(s), dim3(s.loop_blocks), dim3(32 * kLoopWarps),
-                                        s.resident ? rargs : sargs, s.loop_smem, s.st));
-    if (max_steps > lp.slice) AF_CUDA(cudaGraphLaunch(s.exec, s.st));
+    s.rprm.loop.t_stop = t_stop;
+    s.rprm.loop.max_steps = max_steps;
+    AF_TRY(launch_slice(s, 0));
+    const long long n = slices_of(s, (double)max_steps);
+    if (n <= kMaxQueued) {
+      for (long long k = 1; k < n; k++) AF_TRY(launch_slice(s, 1));
+    } else if (wait || !loop_graph(s)) {
+      AF_TRY(finish_slices(s));
+    } else {
+      AF_CUDA(cudaGraphLaunch(s.exec, s.st));
+    }
     return AF_OK;
   }
   if (s.use_cond) {
@@ -1033,7 +1068,7 @@ int af_sim_run(af_sim* h, double t_stop, int64_t max_steps, int64_t* steps_done)
   Sim& s = *h->s;
   AF_TRY(af::read_ctl(s));
   long long before = s.pinned_ctl->step;
-  AF_TRY(af::launch(s, t_stop, max_steps));
+  AF_TRY(af::launch(s, t_stop, max_steps, /*wait=*/true));
   AF_TRY(af::read_ctl(s));
   if (steps_done) *steps_done = s.pinned_ctl->step - before;
   return s.pinned_ctl->status ? AF_ESTATE : AF_OK;

@@ -1,7 +1,7 @@
 // af_stream.cuh -- the time loop of a grid in HBM, many steps in one launch.
 //
 // The strips of af_step.cuh, one cooperative launch for a call's steps, or as
-// many as take some 4 ms: one block per SM, 16 warps, each marching its strips as k_step's
+// many as take some 8 ms: one block per SM, 16 warps, each marching its strips as k_step's
 // one-warp blocks do, and between steps the exchange of af_exchange.cuh instead
 // of a kernel boundary.  A boundary costs its own launch, the last block's fold
 // (a chain of dependent loads and atomics, the rain look-up among them) and

@@ -55,10 +55,11 @@ E2E_TRIALS = 9
 
 
 def loop_launches(cells: int, steps: int) -> int:
-    """Kernels of one call of the streamed FP32 loop: launches of some 4 ms of steps (7 us and 5 us per
-    million cells each, the library's estimate), a one-thread kernel beside each after the first."""
-    per = max(1, int(4000.0 / (7.0 + 5.0e-6 * cells)))
-    return 1 if steps <= per else 2 * -(-steps // per)
+    """Kernels of one call of the streamed FP32 loop that does not wait: launches of some 8 ms of steps
+    (7 us and 5 us per million cells each, the library's estimate), past 16 of them from a graph with a
+    one-thread kernel beside each."""
+    n = -(-steps // max(1, int(8000.0 / (7.0 + 5.0e-6 * cells))))
+    return n if n <= 16 else 2 * n
 
 
 def parse():

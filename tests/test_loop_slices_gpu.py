@@ -68,6 +68,41 @@ def test_other_work_runs_beside_a_long_call(cuda, monkeypatch, mode):
         assert a.steps == 200_010 and float(x[0]) == 6.0
 
 
+@MODES
+def test_other_work_runs_beside_a_call_that_waits(cuda, monkeypatch, mode):
+    with _sim(monkeypatch, mode, _film(700, 600), "f32") as a, _sim(monkeypatch, mode, _film(90, 80), "f32") as b:
+        a.run(1e12, 10)
+        long = threading.Thread(target=a.run, args=(1e12, 100_000))
+        long.start()
+        for _ in range(20):
+            assert b.run(1e12, 50) == 50
+        assert long.is_alive()
+        long.join()
+        assert a.steps == 100_010
+
+
+@MODES
+def test_calls_of_one_to_many_launches_end_where_they_should(cuda, monkeypatch, mode):
+    """Step limits and stop times around the launches of a call, waiting or not."""
+    case = _film(64, 50)
+    with _sim(monkeypatch, mode, case, "f64") as a, _sim(monkeypatch, mode, case, "f64") as b:
+        dt = 0.0
+        for steps in (1, 700, 3000, 9000, 30_000):
+            n0 = a.steps
+            assert a.run(1e12, steps) == steps
+            b.launch(1e12, steps)
+            b.sync()
+            assert a.status() == b.status() and a.steps == n0 + steps
+            dt = a.status()[1]
+            stop = a.t + 0.37 * steps * dt
+            n = a.run(stop)
+            b.launch(stop)
+            b.sync()
+            assert a.status() == b.status() and a.t >= stop and 0 < n < steps + 2
+            assert a.t - a.status()[1] < stop  # no step past the one that reached it
+        np.testing.assert_array_equal(a.depth(), b.depth())
+
+
 def test_two_simulations_in_two_threads(cuda, monkeypatch):
     """Each gets the results it gets alone."""
     cases = [(_film(500, 300, 2), "f32", 6000), (_film(310, 290, 3), "f64", 3000)]
