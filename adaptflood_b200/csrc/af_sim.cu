@@ -851,7 +851,6 @@ static int create(const af_case_desc* c, const af_forcing_desc* f, const double*
   const int nx = c->nx, ny = c->ny;
   s->cells_elems = cell_elems(ny, P);
   s->qy_elems = qy_elems(ny, P);
-  if (const char* e = getenv("AF_PLANE_PAD")) s->qy_elems += (size_t)atoll(e);  // EXPERIMENT
   const size_t plane_bytes = s->qy_elems * s->esize;
   AF_TRY(alloc_field(s->planes, 8 * s->qy_elems, s->esize));
   AF_CUDA(cudaMemsetAsync(s->planes.p, 0, 8 * plane_bytes, s->st));
