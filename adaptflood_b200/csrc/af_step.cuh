@@ -24,7 +24,7 @@
 // uses, so no Qold arrays exist.
 //
 // The strips here run in three kernels: k_step below (one launch a step), the
-// streamed loop (af_stream.cuh: all steps in one launch) and k_batch_step.
+// streamed loop (af_stream.cuh: many steps in one launch) and k_batch_step.
 //
 // Control lives in device memory (SimCtl): time, Hmax, parity, step counters.
 // In k_step the last block to finish (one atomic counter, no waiting) folds Hmax,
@@ -1955,7 +1955,7 @@ const void* step_kernel_f64(int variant, bool tma = true);
 const void* step_kernel_f32(int variant, bool tma = true);
 const void* resident_kernel_f64();  // the resident loop (af_resident.cuh)
 const void* resident_kernel_f32();
-const void* stream_kernel_f64(bool tma);  // the loop in one launch (af_stream.cuh)
+const void* stream_kernel_f64(bool tma);  // the streamed loop (af_stream.cuh)
 const void* stream_kernel_f32(bool tma);
 const void* batch_kernel_f64(int variant);
 const void* batch_kernel_f32(int variant);

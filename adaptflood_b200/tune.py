@@ -13,8 +13,10 @@ R, and returns the fastest R per class (cell-updates/s, CUDA events on the
 batch's stream, after warm-up steps; the better of two timings).  The
 load-adaptive strip height is off while it measures, so each candidate runs
 at its own height (with it on, the taller candidates would be cut down to the
-same height and the choice among them would be noise); a batch that uses
-the tuned heights keeps it on, to lower them when few scenarios remain.  ``tune_variant`` picks the launch
+same height and the choice among them would be noise).  A batch needs no
+tuned heights: before each launch it estimates one height for its members, of up
+to 32 rows; heights that are set are upper limits of that, or, with the
+balance at 0, the heights themselves.  ``tune_variant`` picks the launch
 shape (warps per block x resident blocks per SM) of the batch kernel the
 same way.  Results do not depend on R or the variant (bit for bit), only
 the speed does.
