@@ -493,7 +493,6 @@ static double* stage_of(Sim& s, int par, size_t& cap) {
   return static_cast<double*>(s.Qx[par ^ 1].p);
 }
 static int clear_stage(Sim& s, double* stage, size_t cap, int rows, int width) {
-  if (s.prec == AF_PREC_F64 && direct_rows(width)) return AF_OK;
   AF_CUDA(cudaMemsetAsync(stage, 0, std::min(cap, (size_t)rows * width * 8), s.st));
   return AF_OK;
 }
@@ -505,7 +504,8 @@ static int put_field(Sim& s, int par, DevBuf& b, const double* src, int rows, in
   AF_TRY(s.prec == AF_PREC_F64
              ? put_rows(s.buf<double>(b), s.P, src, rows, width, hpitch, stage, cap, s.st)
              : put_rows(s.buf<float>(b), s.P, src, rows, width, hpitch, stage, cap, s.st));
-  AF_TRY(clear_stage(s, stage, cap, rows, width));
+  if (s.prec == AF_PREC_F32 || !direct_rows(width))
+    AF_TRY(clear_stage(s, stage, cap, rows, width));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }
@@ -517,7 +517,8 @@ static int get_field(Sim& s, int par, DevBuf& b, double* dst, int rows, int widt
   AF_TRY(s.prec == AF_PREC_F64
              ? get_rows(s.buf<double>(b), s.P, dst, rows, width, hpitch, stage, cap, s.st)
              : get_rows(s.buf<float>(b), s.P, dst, rows, width, hpitch, stage, cap, s.st));
-  AF_TRY(clear_stage(s, stage, cap, rows, width));
+  if (s.prec == AF_PREC_F32 || !direct_back(rows, width))
+    AF_TRY(clear_stage(s, stage, cap, rows, width));
   AF_CUDA(cudaStreamSynchronize(s.st));
   return AF_OK;
 }

@@ -189,6 +189,16 @@ constexpr size_t kStageBytes = 64u << 20;
 // FP64 rows at least this long go straight into the padded field.
 constexpr size_t kLongRow = 16384;
 inline bool direct_rows(int width) { return (size_t)width * 8 >= kLongRow; }
+// And so do small FP64 fields on their way back, which the copy engine has moved
+// before a kernel and a copy would have: of rows of whole 32 bytes up to 2048, of
+// others, which it moves more slowly, up to 128.  us for a depth field, straight / by
+// way of the buffer: 20x32 27 / 39, 20x2000 65 / 66, 200x600 92 / 110, 1000x128 (1 MB)
+// 95 / 105, 2000x128 410 / 160; 101x129 51 / 52, 101x300 83 / 59, 317x203 99 / 82.  (To
+// the device both take the same.)
+inline bool direct_back(int rows, int width) {
+  return direct_rows(width) || (rows <= (width % 4 == 0 ? 2048 : 128) &&
+                                (size_t)rows * width * 8 <= (1u << 20));
+}
 
 template <typename T>
 __global__ void k_pad_from_f64(const double* __restrict__ src, int rows, int width,
@@ -238,7 +248,7 @@ int put_rows(T* dst, int P, const double* src, int rows, int width, size_t hpitc
 template <typename T>
 int get_rows(const T* src, int P, double* dst, int rows, int width, size_t hpitch, double* stage,
              size_t cap, cudaStream_t st) {
-  if (sizeof(T) == 8 && direct_rows(width)) {
+  if (sizeof(T) == 8 && direct_back(rows, width)) {
     AF_CUDA(copy2d_d2h(dst, hpitch * 8, src, (size_t)P * 8, (size_t)width * 8, rows, st));
     return AF_OK;
   }
