@@ -211,7 +211,10 @@ int af_sim_destroy(af_sim* s);
 /* Enqueues steps while t < t_stop and fewer than max_steps steps have run in
  * this call (the loop test of src/main.cpp:227), without waiting.  The steps
  * take the whole GPU for some milliseconds at a time; work on other streams (another
- * simulation, a batch, the caller's kernels) runs in between. */
+ * simulation, a batch, the caller's kernels) runs in between.  Simulations that
+ * run at once so share the GPU in time: many small grids belong in a batch, or are
+ * created with AF_SIM_LOOP=graph in the environment, which launches a kernel per
+ * step that leaves room beside it (slower for one). */
 int af_sim_launch(af_sim* s, double t_stop, int64_t max_steps);
 /* Waits for the enqueued steps. */
 int af_sim_sync(af_sim* s);
